@@ -103,6 +103,7 @@ def lib() -> C.CDLL:
     L.sf_get_counters.argtypes = [C.c_char_p, C.POINTER(C.c_int64), C.c_int32]
     L.sfb200_debug_force_token_tile.argtypes = [i]
     L.sfb200_debug_plan_gemm.argtypes = [i, i, i, i, i]
+    L.sfb200_debug_route_gemm.argtypes = [i, i, i, i, i]
     L.sfb200_debug_pair_tuning.argtypes = [i, i]
     L.sfb200_debug_host_pipeline.argtypes = [i, i]
     L.sfb200_debug_host_chunk_plan.argtypes = [i, i, i, C.POINTER(C.c_int)]

@@ -375,7 +375,7 @@ int sfb200_sparse_gemm_scatter(const void* x, int ldx, const void* values, const
   a.tok_per_owner = tok_per_owner;
   // a forced variant of another kernel family means nothing here: let the pair launcher choose (it keeps to the tiles
   // with two accumulator sets, whose drain -- here stores over NVLink -- hides behind the next tile's K loop)
-  if (a.force_bn < 1000 || (a.force_bn >= 3000 && a.force_bn < 5000)) a.force_bn = 0;
+  if (a.force_bn < 1000 || (a.force_bn >= 3000 && a.force_bn < 5000) || a.force_bn >= 6000) a.force_bn = 0;
   return launch_sparse_gemm_pair(a, static_cast<cudaStream_t>(stream));
 }
 
@@ -476,11 +476,17 @@ SFB200_API int sfb200_debug_pair_tuning(int l2_band_mb, int force_order) {
   return kOk;
 }
 
-/* Which kernel variant sfb200_sparse_gemm (swiglu = 0) or sfb200_sparse_gemm_swiglu (swiglu = 1, N = 2 * I
- * rows) runs for a shape on a GPU with num_sms SMs, in the numbering of sfb200_debug_force_token_tile.  Host-only. */
+/* The variant for a shape among the kernels of fixed tiles, and the one sfb200_sparse_gemm (swiglu = 0) or
+ * sfb200_sparse_gemm_swiglu (swiglu = 1, N = 2 * I rows) runs: the same, or a form of the band kernel (6000 / 7000 + token
+ * tile).  On a GPU with num_sms SMs, in the numbering of sfb200_debug_force_token_tile.  Host-only. */
 SFB200_API int sfb200_debug_plan_gemm(int M, int N, int K, int swiglu, int num_sms) {
   if (M <= 0 || N <= 0 || K <= 0 || num_sms <= 0) return 0;
   return plan_sparse_gemm(M, N, K, swiglu ? kEpiSwiGLU : kEpiStore, num_sms);
+}
+
+SFB200_API int sfb200_debug_route_gemm(int M, int N, int K, int swiglu, int num_sms) {
+  if (M <= 0 || N <= 0 || K <= 0 || num_sms <= 0) return 0;
+  return route_sparse_gemm(M, N, K, swiglu ? kEpiSwiGLU : kEpiStore, num_sms);
 }
 
 /* The chunk plan sfb200_ffn_forward_host would use for M tokens (host-only; out8 holds 8 ints). */

@@ -363,7 +363,7 @@ int launch_cfg(const SparseGemmArgs& a, cudaStream_t stream) {
 // Measured on B200 (variants timed as CUDA graphs against this model): 22016 x 4096 at 1024 tokens 112 -> 88 us with the
 // 256 x 208 pair tile; 4096 x 11008 at 1024 tokens stays with the single-CTA 256-token tile (32 row tiles x 4 = 128 tiles
 // = one wave on 148 SMs, 59.6 us, against two waves of pair tiles, 66 us).
-int pick_mid_variant(int n_out, int m_tok, int K, int num_sms, int swiglu) {
+int pick_mid_variant(int n_out, int m_tok, int K, int num_sms, int swiglu, double* cost_us = nullptr) {
   const double k64 = (K + 63) / 64;
   const long mb = (n_out + 127) / 128;
   double best = 1e30;
@@ -380,7 +380,11 @@ int pick_mid_variant(int n_out, int m_tok, int K, int num_sms, int swiglu) {
   }
   double pcost = 1e30;
   const int pv = pick_pair_variant(n_out, m_tok, K, num_sms, swiglu, &pcost);
-  if (pcost < 0.97 * best) pick = pv;
+  if (pcost < 0.97 * best) {
+    pick = pv;
+    best = pcost;
+  }
+  if (cost_us) *cost_us = best;
   return pick;
 }
 
@@ -428,6 +432,23 @@ int plan_sparse_gemm(int m_tok, int n_out, int K, int epi, int num_sms) {
   return pick_mid_variant(n_out, m_tok, K, num_sms, epi == kEpiSwiGLU);
 }
 
+// From 65 to 1023 tokens the band kernel (sparse_gemm_sm100_band.cu) is weighed against the fixed tiles.  Up to 160 tokens
+// it is taken outright: measured on 22016, 28672, 11008, 57344 x 4096 / 8192 and 4096, 8192, 2048-row weights it is 1.0-1.9 x
+// the fixed choice there (4096 x 11008 at 150 tokens 34.6 -> 18.5 us, 22016 x 4096 at 150 tokens 32.8 -> 27.1 us, 4096 x 4096
+// at 100 tokens 11.4 -> 11.3 us); above, the lower estimate decides (300 tokens: 34.4 -> 22.9 and 42.1 -> 34.8 us; 512
+// tokens: 34.9 -> 28.1 and 52.7 -> 47.1 us; at 700 tokens the two meet).  At 64 tokens and below a stage of the single-CTA
+// kernels carries as few token bytes as a pair's and their split-K form uses 128 SMs: 13.8 against 16.1 us on 4096 x 11008
+// at 24 tokens.
+int route_sparse_gemm(int m_tok, int n_out, int K, int epi, int num_sms) {
+  const int fixed = plan_sparse_gemm(m_tok, n_out, K, epi, num_sms);
+  if (m_tok <= 64 || m_tok >= kPairMinTokens) return fixed;
+  double band_us = 0.0, fixed_us = 0.0;
+  const int band = pick_band_variant(m_tok, n_out, K, num_sms, &band_us);
+  if (m_tok <= 160) return band;
+  pick_mid_variant(n_out, m_tok, K, num_sms, epi == kEpiSwiGLU, &fixed_us);
+  return band_us < fixed_us ? band : fixed;
+}
+
 int launch_sparse_gemm(const SparseGemmArgs& a, cudaStream_t stream) {
   if (a.K % 64 != 0 || a.K <= 0 || a.m_tok <= 0 || a.n_out <= 0) return kErrInvalid;
   if (a.n_out % 8 != 0 || a.ldx % 8 != 0 || a.ldy % 8 != 0) return kErrInvalid;
@@ -439,13 +460,14 @@ int launch_sparse_gemm(const SparseGemmArgs& a, cudaStream_t stream) {
   if (a.out_f32) {
     // fp32 output exists in the CTA-pair kernel's epilogue only
     if (a.epi != kEpiStore) return kErrInvalid;
-    if (b.force_bn < 1000 || (b.force_bn >= 3000 && b.force_bn < 5000))
+    if (b.force_bn < 1000 || (b.force_bn >= 3000 && b.force_bn < 5000) || b.force_bn >= 6000)
       b.force_bn = pick_pair_variant(a.n_out, a.m_tok, a.K, a.num_sms, 0);
     return launch_sparse_gemm_pair(b, stream);
   }
-  if (b.force_bn == 0) b.force_bn = plan_sparse_gemm(a.m_tok, a.n_out, a.K, a.epi, a.num_sms);
+  if (b.force_bn == 0) b.force_bn = route_sparse_gemm(a.m_tok, a.n_out, a.K, a.epi, a.num_sms);
   const int v = b.force_bn;
   if (v == 8) return launch_sparse_gemm_small_m(b, stream);
+  if (v >= 6000) return launch_sparse_gemm_band(b, stream);
   if (v >= 5000) return launch_sparse_gemm_pair(b, stream);
   if (v >= 3000) return launch_sparse_gemm_splitk(b, v >= 4000 ? 4 : 2, stream);
   if (v >= 1000) return launch_sparse_gemm_pair(b, stream);
