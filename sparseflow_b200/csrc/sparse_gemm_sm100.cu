@@ -21,6 +21,7 @@
 #include <stdint.h>
 
 #include "kernels.h"
+#include "launch.h"
 #include "sm100_ptx.cuh"
 #include "tensor_map.h"
 
@@ -130,6 +131,13 @@ sparse_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
     tma_prefetch_desc(&tmB);
     tma_prefetch_desc(&tmD);
   }
+  if (threadIdx.x == 64) {      // the first ring of weight tiles into L2, under the previous kernel's tail
+    const int m_blk = blockIdx.x / p.num_n_blks;
+    for (int kt = 0; kt < k_iters && kt < C::STAGES; ++kt) {
+      prefetch_l2_2d(&tmA, kt * (C::BK / 2), m_blk * C::BM);
+      if (C::BK == 128) prefetch_l2_bulk(p.meta + (static_cast<size_t>(m_blk) * p.k_tiles128 + kt) * 512, C::E_BYTES);
+    }
+  }
   if (warp == 1) {
     tmem_alloc(smem_u32(tmem_slot), C::TMEM_COLS);
     tmem_relinquish();
@@ -138,6 +146,8 @@ sparse_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  dependency_wait();
+  dependency_trigger();
 
   if (warp == 0) {
     // ------------------------------------------------------------ TMA producer
@@ -349,8 +359,7 @@ int launch_cfg(const SparseGemmArgs& a, cudaStream_t stream) {
   const int tiles = p.num_m_blks * p.num_n_blks;
   int grid = a.num_sms < tiles ? a.num_sms : tiles;
   if (grid < 1) grid = 1;
-  sparse_gemm_kernel<C><<<grid, 192, C::SMEM_BYTES, stream>>>(tmA, tmB, tmD, p);
-  return cudaGetLastError() == cudaSuccess ? kOk : kErrCuda;
+  return launch_dependent(sparse_gemm_kernel<C>, grid, 192, C::SMEM_BYTES, 0, stream, tmA, tmB, tmD, p);
 }
 
 // Kernel / token-tile choice from 129 tokens up: the cheapest, by estimated time, of the single-CTA tiles and the

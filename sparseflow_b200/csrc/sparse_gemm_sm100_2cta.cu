@@ -28,6 +28,7 @@
 #include <stdint.h>
 
 #include "kernels.h"
+#include "launch.h"
 #include "sm100_pair.cuh"
 #include "sm100_ptx.cuh"
 #include "tensor_map.h"
@@ -212,9 +213,19 @@ __device__ __forceinline__ void pair_kernel_body(const CUtensorMap& tmA, const C
       mbar_init(bar_acce + 8 * b, 2 * C::EPI_WARPS);
     }
     mbar_fence_init();
-    tma_prefetch_desc(&tmA);
     tma_prefetch_desc(&tmB);
-    tma_prefetch_desc(&tmE);
+  }
+  if (threadIdx.x == 64) {      // the first ring of weight tiles into L2, under the previous kernel's tail
+    int m_blk, n_blk;
+    tile_coords(pair_id, p, m_blk, n_blk);
+    const int row0 = m_blk * C::ROWS_TILE + static_cast<int>(rank) * C::ROWS_CTA;
+    for (int kt = 0; kt < k_iters && kt < C::STAGES; ++kt)
+#pragma unroll
+      for (int rs = 0; rs < C::RS; ++rs) {
+        if (row0 + 128 * rs >= p.n_out) break;
+        prefetch_l2_2d(&tmA, kt * (C::BK / 2), row0 + 128 * rs);
+        if (C::BK == 128) prefetch_l2_1d_tensor(&tmE, (((row0 >> 7) + rs) * p.k_tiles128 + kt) * 256);
+      }
   }
   if (warp == 1) {
     tmem_alloc_pair(smem_u32(tmem_slot), C::TMEM_COLS);
@@ -225,6 +236,8 @@ __device__ __forceinline__ void pair_kernel_body(const CUtensorMap& tmA, const C
   cluster_sync_all();   // both CTAs' barriers are initialised before anything remote touches them
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  dependency_wait();
+  dependency_trigger();
 
   if (warp == 0) {
     // ------------------------------------------------------------ TMA producer (both CTAs)
@@ -593,8 +606,7 @@ int launch_pair_cfg(const SparseGemmArgs& a, cudaStream_t stream) {
   int pairs = a.num_sms / 2;
   if (pairs > tiles) pairs = tiles;
   if (pairs < 1) pairs = 1;
-  sparse_gemm_pair_kernel<C><<<2 * pairs, C::THREADS, C::SMEM_BYTES, stream>>>(tmA, tmB, tmE, p);
-  return cudaGetLastError() == cudaSuccess ? kOk : kErrCuda;
+  return launch_dependent(sparse_gemm_pair_kernel<C>, 2 * pairs, C::THREADS, C::SMEM_BYTES, 0, stream, tmA, tmB, tmE, p);
 }
 
 // Tile choice among the variants of dispatch_pair: estimated kernel time in microseconds from measurements on B200.

@@ -31,6 +31,7 @@
 #include <cmath>
 
 #include "kernels.h"
+#include "launch.h"
 #include "sm100_pair.cuh"
 #include "sm100_ptx.cuh"
 #include "tensor_map.h"
@@ -156,10 +157,18 @@ sparse_gemm_band_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_co
       mbar_init(bar_acce + 8 * b, 2 * kEpiWarps);
     }
     mbar_fence_init();
-    tma_prefetch_desc(&tmA);
     tma_prefetch_desc(&tmB);
     tma_prefetch_desc(&tmBt);
-    tma_prefetch_desc(&tmE);
+  }
+  if (threadIdx.x == 64) {      // the first ring of weight tiles into L2, under the previous kernel's tail
+    Item it;
+    if (items > 0 && get_item(0, cluster_id, num_clusters, p, it)) {
+      const int row0 = it.m_blk * 256 + static_cast<int>(rank) * 128, e_row = (row0 >> 7) * p.k_tiles128;
+      for (int kt = k_begin; row0 < p.n_out && kt < k_end && kt < k_begin + p.stages; ++kt) {
+        prefetch_l2_2d(&tmA, kt * 64, row0);
+        prefetch_l2_1d_tensor(&tmE, (e_row + kt) * 256);
+      }
+    }
   }
   if (warp == 1) {
     tmem_alloc_pair(smem_u32(tmem_slot), p.tmem_cols);
@@ -169,6 +178,8 @@ sparse_gemm_band_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_co
   __syncthreads();
   cluster_sync_all();   // every CTA's barriers are initialised before anything remote touches them
   tc_fence_after();
+  dependency_wait();
+  dependency_trigger();
   const uint32_t tmem_base = *tmem_slot;
 
   if (warp == 0) {
@@ -479,23 +490,9 @@ int launch_band(const SparseGemmArgs& a, int split, int t, cudaStream_t stream) 
   // split > 1: one cluster per tile; split 1: persistent pairs (a plan with slices fills whole passes before them)
   const int work = p.n_full > 0 ? p.n_full : p.n_tail;
   const int clusters = (split > 1 || work < pairs) ? work : pairs;
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(static_cast<unsigned>(clusters * 2 * split), 1, 1);
-  cfg.blockDim = dim3(kThreads, 1, 1);
-  cfg.dynamicSmemBytes = 1024 + p.stages * stage_bytes(t) + kEpiWarps * kStagingBytes + kBarBytes;
-  cfg.stream = stream;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = static_cast<unsigned>(2 * split);
-  attr[0].val.clusterDim.y = 1;
-  attr[0].val.clusterDim.z = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  if (cudaLaunchKernelEx(&cfg, sparse_gemm_band_kernel<EPI>, tmA, tmB, tmBt, tmE, p) != cudaSuccess) {
-    cudaGetLastError();
-    return kErrCuda;
-  }
-  return kOk;
+  const size_t smem = 1024 + p.stages * stage_bytes(t) + kEpiWarps * kStagingBytes + kBarBytes;
+  return launch_dependent(sparse_gemm_band_kernel<EPI>, clusters * 2 * split, kThreads, smem, 2 * split, stream, tmA, tmB, tmBt,
+                          tmE, p);
 }
 
 // Estimated time in us of one (split, token tile) on a GPU with num_sms SMs; constants measured on B200.

@@ -19,6 +19,7 @@
 #include <stdint.h>
 
 #include "kernels.h"
+#include "launch.h"
 #include "sm100_ptx.cuh"
 #include "tensor_map.h"
 
@@ -110,8 +111,13 @@ sparse_gemm_splitk_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_
     }
     mbar_init(bar_accf, 1);
     mbar_fence_init();
-    tma_prefetch_desc(&tmA);
     tma_prefetch_desc(&tmB);
+  }
+  if (threadIdx.x == 64) {      // the first ring of weight tiles into L2, under the previous kernel's tail
+    for (int kt = kt_begin; kt < kt_end && kt < kt_begin + C::STAGES; ++kt) {
+      prefetch_l2_2d(&tmA, kt * (C::BK / 2), m_blk * C::BM);
+      prefetch_l2_bulk(p.meta + (static_cast<size_t>(m_blk) * p.k_tiles128 + kt) * 512, C::E_BYTES);
+    }
   }
   if (warp == 1) {
     tmem_alloc(smem_u32(tmem_slot), C::TMEM_COLS);
@@ -121,6 +127,8 @@ sparse_gemm_splitk_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  dependency_wait();
+  dependency_trigger();
   // First cluster barrier, split: arrive now, wait only before the first store into a peer's slots
   // (its purpose is that every CTA of the cluster is resident by then), so the K loop does not pay for it.
   cluster_arrive();
@@ -286,23 +294,7 @@ int launch_sk(const SparseGemmArgs& a, int split, cudaStream_t stream) {
   p.fmt = a.fmt;
   p.act = a.act;
   const int tiles = ((a.n_out + C::BM - 1) / C::BM) * p.num_n_blks;
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(static_cast<unsigned>(tiles * split), 1, 1);
-  cfg.blockDim = dim3(192, 1, 1);
-  cfg.dynamicSmemBytes = C::SMEM_BYTES;
-  cfg.stream = stream;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = static_cast<unsigned>(split);
-  attr[0].val.clusterDim.y = 1;
-  attr[0].val.clusterDim.z = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  if (cudaLaunchKernelEx(&cfg, sparse_gemm_splitk_kernel<C>, tmA, tmB, p) != cudaSuccess) {
-    cudaGetLastError();
-    return kErrCuda;
-  }
-  return kOk;
+  return launch_dependent(sparse_gemm_splitk_kernel<C>, tiles * split, 192, C::SMEM_BYTES, split, stream, tmA, tmB, p);
 }
 
 }  // namespace

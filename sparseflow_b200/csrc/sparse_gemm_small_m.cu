@@ -25,6 +25,8 @@
 #include <stdint.h>
 
 #include "kernels.h"
+#include "launch.h"
+#include "sm100_ptx.cuh"
 
 namespace sfb200 {
 namespace {
@@ -107,6 +109,21 @@ __global__ void __launch_bounds__(kWarps * 32) sparse_gemm_small_m_kernel(const 
   const int kt_hi = (p.k_tiles128 * (warp + 1)) / kWarps;
   const int n_kt = kt_hi - kt_lo;
   const int kc_total = p.K / 2;   // compressed elements per row
+
+  // the first ring of this warp's weight slices into L2, under the previous kernel's tail (128 contiguous bytes per row
+  // and K tile, 256 of metadata)
+  for (int i = 0; i < kStages && i < n_kt; ++i) {
+    const int row = static_cast<int>(blockIdx.x) * kRows + lane;
+    if (lane < kRows && row < p.n_out)
+      prefetch_l2_line(p.values + static_cast<size_t>(row) * kc_total + (kt_lo + i) * 64);
+    if (lane < 2 * SL) {
+      const int r16 = static_cast<int>(blockIdx.x) * kRows + 16 * (lane >> 1);
+      prefetch_l2_line(p.meta + ((static_cast<size_t>(r16 >> 7) * p.k_tiles128 + kt_lo + i) * 128 + ((r16 & 127) >> 4) * 16 +
+                                 8 * (lane & 1)) * 4);
+    }
+  }
+  dependency_wait();
+  dependency_trigger();
 
   // X fragment cache of this warp's K slice: xs[(k-step * NT + n) * 32 + lane] = (b0, b1, b2, b3)
   uint4* xs = nullptr;
@@ -315,9 +332,7 @@ int launch_nt(SmallParams p, int num_sms, cudaStream_t stream) {
   const bool two = smem <= 110 * 1024 && 2 * r2 <= r1;
   long ctas = static_cast<long>(num_sms) * (two ? 2 : 1);
   if (ctas > units) ctas = units;
-  sparse_gemm_small_m_kernel<NT, SL, SWIGLU, BF16>
-      <<<static_cast<int>(ctas), kWarps * 32, smem, stream>>>(p);
-  return cudaGetLastError() == cudaSuccess ? kOk : kErrCuda;
+  return launch_dependent(sparse_gemm_small_m_kernel<NT, SL, SWIGLU, BF16>, static_cast<int>(ctas), kWarps * 32, smem, 0, stream, p);
 }
 
 template <int SL, bool SWIGLU>
