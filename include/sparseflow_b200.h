@@ -304,7 +304,8 @@ SFB200_API int sfb200_debug_pair_tuning(int l2_band_mb, int force_order);
 
 /* For Y[M, N] = X[M, K] . W^T (swiglu = 1: the fused gate|up GEMM, N = 2 * I rows) on a GPU with num_sms SMs, in the
  * numbering above; 0 for a non-positive size.  Host-only.  _plan_gemm: the choice among the kernels of fixed tiles;
- * _route_gemm: what a call with nothing forced runs, that choice or a 6000 / 7000 form where it is faster. */
+ * _route_gemm: what a call with nothing forced runs: that choice, a 6000 / 7000 form where it is faster, or a 512-row pair
+ * tile in place of a 256-row one where that is faster at the power limit. */
 SFB200_API int sfb200_debug_plan_gemm(int M, int N, int K, int swiglu, int num_sms);
 SFB200_API int sfb200_debug_route_gemm(int M, int N, int K, int swiglu, int num_sms);
 

@@ -87,6 +87,8 @@ void set_pair_tuning(int l2_band_mb, int force_order);
 // Variant the CTA-pair launcher picks on its own (1192..1256 or 5192..5240; swiglu: the SiLU.mul epilogue) and,
 // optionally, its estimated time in us.
 int pick_pair_variant(int n_out, int m_tok, int K, int num_sms, int swiglu, double* cost_us = nullptr);
+// The same with a preference for the 512-row tiles, which need less energy.
+int pick_pair_variant_sustained(int n_out, int m_tok, int K, int num_sms, int swiglu);
 // The kernel variant for a shape among the kernels of fixed tiles, in the numbering of
 // SparseGemmArgs::force_bn: 8 decode kernel; 32..256 single-CTA kernel with that token tile; 1192..1256 / 5192..5240
 // CTA-pair kernel; 3000 + tile / 4000 + tile split-K cluster kernel with 2 / 4 K slices.  Host-only.
@@ -125,8 +127,8 @@ int splitk_token_tile(int m_tok);
 int launch_sparse_gemm_band(const SparseGemmArgs& a, cudaStream_t stream);
 // The form of that kernel estimated fastest for a shape (6000 + t or 7000 + t) and its estimated time in us.
 int pick_band_variant(int m_tok, int n_out, int K, int num_sms, double* cost_us = nullptr);
-// What launch_sparse_gemm runs for a 16-bit result when nothing is forced: the band form where it is the faster one, else
-// plan_sparse_gemm's choice among the fixed tiles.  Host-only.
+// What launch_sparse_gemm runs for a 16-bit result when nothing is forced: the band form where it is the faster one, a
+// 512-row pair tile where that needs less energy, else plan_sparse_gemm's choice among the fixed tiles.  Host-only.
 int route_sparse_gemm(int m_tok, int n_out, int K, int epi, int num_sms);
 
 // ---- small-M (decode) sparse GEMM ----------------------------------------------------------

@@ -450,6 +450,8 @@ int plan_sparse_gemm(int m_tok, int n_out, int K, int epi, int num_sms) {
 // at 24 tokens.
 int route_sparse_gemm(int m_tok, int n_out, int K, int epi, int num_sms) {
   const int fixed = plan_sparse_gemm(m_tok, n_out, K, epi, num_sms);
+  if (m_tok >= kPairMinTokens && fixed >= 1192 && fixed <= 1240)
+    return pick_pair_variant_sustained(n_out, m_tok, K, num_sms, epi == kEpiSwiGLU);
   if (m_tok <= 64 || m_tok >= kPairMinTokens) return fixed;
   double band_us = 0.0, fixed_us = 0.0;
   const int band = pick_band_variant(m_tok, n_out, K, num_sms, &band_us);

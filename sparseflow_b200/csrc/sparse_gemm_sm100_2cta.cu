@@ -625,7 +625,8 @@ int launch_pair_cfg(const SparseGemmArgs& a, cudaStream_t stream) {
 //     the others need two (4096 x 11008 at 1024 tokens: 64 tiles, 46 us against 64 us for the next best);
 //   launch, prologue, first fill and last drain: 8.5 us.
 // What decides in practice is the number of passes over the SM pairs.
-int pick_pair_variant_impl(int n_out, int m_tok, int K, int pairs, int swiglu, double* cost_us, bool hidden_drain = false) {
+int pick_pair_variant_impl(int n_out, int m_tok, int K, int pairs, int swiglu, double* cost_us, bool hidden_drain = false,
+                           double bias512 = 0.98) {
   const double k128 = (K + 127) / 128;
   const double dbl = k128 > 32.0 ? std::log2(k128 / 32.0) : 0.0;
   const double fk = 1.0 + 0.08 * (dbl < 1.5 ? dbl : 1.5);
@@ -656,7 +657,7 @@ int pick_pair_variant_impl(int n_out, int m_tok, int K, int pairs, int swiglu, d
       const double c = 8.5 + waves(t2) * (k128 * (0.247 + 0.00199 * bn) * crowd + (swiglu ? 1.5 : 4.0));
       if (c < c5 * 0.985) { c5 = c; b5 = 5000 + bn; }
     }
-    if (c5 < best_cost * 0.98) { best_cost = c5; best = b5; }
+    if (c5 < best_cost * bias512) { best_cost = c5; best = b5; }
   }
   if (cost_us) *cost_us = best_cost;
   return best;
@@ -695,6 +696,17 @@ void set_pair_tuning(int l2_band_mb, int force_order) {
 
 int pick_pair_variant(int n_out, int m_tok, int K, int num_sms, int swiglu, double* cost_us) {
   return pick_pair_variant_impl(n_out, m_tok, K, num_sms / 2 > 0 ? num_sms / 2 : 1, swiglu, cost_us);
+}
+
+// What launch_sparse_gemm takes among the pair tiles.  The estimates above are times at full clock; a GPU that does this
+// work for longer than a few milliseconds runs at its power limit, where time follows energy, and a 512-row tile moves 14 %
+// fewer bytes through shared memory and 31 % fewer through L2 per flop than a 256-row one.  So a 512-row tile is taken up to
+// an estimate 6 % above the best.  Measured at the power limit (22016 x 4096 at 4096 / 8192 tokens 337 -> 321 / 660 -> 626 us,
+// 11008 x 4096 at 2048 / 3000 tokens 95.8 -> 91.4 / 133.7 -> 128.6 us, 4096 x 4096 at 1500 / 4096 / 8192 tokens 32.1 -> 30.2 /
+// 69.5 -> 67.6 / 131.3 -> 126.5 us), on 52 shapes from 1024 tokens: 0.1 % above the best variant on average (0.9 % without),
+// none more than 0.5 % slower; in short bursts at full clock the tiles within 6 % are about equal.
+int pick_pair_variant_sustained(int n_out, int m_tok, int K, int num_sms, int swiglu) {
+  return pick_pair_variant_impl(n_out, m_tok, K, num_sms / 2 > 0 ? num_sms / 2 : 1, swiglu, nullptr, false, 1.06);
 }
 
 int launch_sparse_gemm_pair(const SparseGemmArgs& a, cudaStream_t stream) {

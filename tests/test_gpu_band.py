@@ -14,7 +14,8 @@ def _route(M, N, K, sw=0, sms=148):
 
 
 def test_route_takes_known_forms():
-    """Band forms only from 65 to 1023 tokens, with a legal tile; everything else is the fixed-tile plan."""
+    """Band forms only from 65 to 1023 tokens, with a legal tile; from 1024 tokens a 256-row pair tile may give way to a
+    512-row one; everything else is the fixed-tile plan."""
     plan = _lib.lib().sfb200_debug_plan_gemm
     for sms in (148, 132, 64, 2):
         for N, K in ((4096, 4096), (22016, 4096), (4096, 11008), (57344, 8192), (8, 64), (392, 1088), (1024, 512)):
@@ -24,8 +25,11 @@ def test_route_takes_known_forms():
                     t = v % 1000
                     assert 64 < M < 1024 and v < 8000 and 16 <= t <= 256 and t % 16 == 0, (M, N, K, sms, v)
                     assert v < 7000 or K >= 1024 - 127, (M, N, K, sms, v)
+                elif M >= 1024 and 1192 <= plan(M, N, K, 0, sms) <= 1240:
+                    assert v in (1192, 1208, 1224, 1240, 5192, 5208, 5224, 5240), (M, N, K, sms, v)
                 else:
                     assert v == plan(M, N, K, 0, sms) and not 64 < M <= 160, (M, N, K, sms, v)
+    assert _route(4096, 22016, 4096, 1) == 5240 and _route(1500, 4096, 4096) == 5192
     assert _route(150, 4096, 11008) == 7080 and _route(150, 22016, 4096, 1) == 6160 and _route(0, 8, 64) == 0
 
 
