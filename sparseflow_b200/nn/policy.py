@@ -7,8 +7,16 @@ the B200 crossovers of the measured gate table (``gate_sm100.json``, see ``dispa
 the reference's A100 numbers, and each op class has a second, low band ``M <= decode_max_M_*`` in which
 the sparse path wins because it streams 0.5625x the weight bytes (0 = no such band)."""
 from dataclasses import dataclass, field
+from functools import lru_cache
 
 from .. import dispatch as _gate
+
+
+@lru_cache(maxsize=None)
+def _sm_major(device: int) -> int:
+    """Compute-capability major of a CUDA device: fixed for the life of the process, and asked for on every forward."""
+    import torch
+    return torch.cuda.get_device_capability(device)[0]
 
 
 def _lo(cls):
@@ -53,8 +61,7 @@ class SparseFlowPolicy:
         import torch
         if not torch.cuda.is_available():
             return False
-        major, _ = torch.cuda.get_device_capability()
-        return major == 10
+        return _sm_major(torch.cuda.current_device()) == 10
 
     # which pair of fields an op name of a policy file sets: first match wins, in the order upstream tests them
     # (sparseflow/nn/policy.py:37-72): "gate"/"up" anywhere in the name, then "down", then q/k/v_proj, then any "o"

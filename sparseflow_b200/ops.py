@@ -187,13 +187,13 @@ def _kernel_ready(x: torch.Tensor) -> torch.Tensor:
 
 def _check_bias(bias: torch.Tensor, x: torch.Tensor, rows: int) -> torch.Tensor:
     """The epilogue reads `rows` bias values in the GEMM's own 16-bit type."""
-    if not bias.is_cuda or bias.device != x.device:
+    if not bias.is_cuda or bias.get_device() != x.get_device():
         raise ValueError(f"bias must be a CUDA tensor on {x.device}, got {bias.device}")
     if bias.dtype != x.dtype:
         raise ValueError(f"bias dtype {bias.dtype} != activation dtype {x.dtype}")
     if bias.numel() != rows:
         raise ValueError(f"bias has {bias.numel()} elements, weight has {rows} rows")
-    return bias.contiguous().view(-1)
+    return bias if bias.is_contiguous() else bias.contiguous()
 
 
 def sparse_gemm(x: torch.Tensor, cw: Compressed24, bias: Optional[torch.Tensor] = None,
@@ -208,15 +208,17 @@ def sparse_gemm(x: torch.Tensor, cw: Compressed24, bias: Optional[torch.Tensor] 
     if bias is not None:
         bias = _check_bias(bias, x, cw.rows)
     M = x.shape[0]
-    with _on(x.device):
+    dev = x.get_device()
+    with _NO_SWITCH if dev == torch.cuda.current_device() else torch.cuda.device(dev):
         if out is None:
-            out = torch.empty((M, cw.rows), dtype=x.dtype, device=x.device)
+            out = x.new_empty((M, cw.rows))
         if M == 0:                      # empty batch: nothing to launch
             return out
         rc = _lib.lib().sfb200_sparse_gemm(x.data_ptr(), x.stride(0), cw.values.data_ptr(),
                                            cw.meta.data_ptr(), out.data_ptr(), out.stride(0), M, cw.rows,
                                            cw.K, _dt(x), _ptr(bias), ACT[act], _stream())
-    _lib.check("sfb200_sparse_gemm", rc)
+    if rc:
+        _lib.check("sfb200_sparse_gemm", rc)
     return out
 
 
@@ -229,15 +231,17 @@ def sparse_gemm_swiglu(x: torch.Tensor, cw_gu: Compressed24, out: Optional[torch
         raise ValueError("shape / dtype mismatch")
     x = _kernel_ready(x)
     M, I = x.shape[0], cw_gu.rows // 2
-    with _on(x.device):
+    dev = x.get_device()
+    with _NO_SWITCH if dev == torch.cuda.current_device() else torch.cuda.device(dev):
         if out is None:
-            out = torch.empty((M, I), dtype=x.dtype, device=x.device)
+            out = x.new_empty((M, I))
         if M == 0:
             return out
         rc = _lib.lib().sfb200_sparse_gemm_swiglu(x.data_ptr(), x.stride(0), cw_gu.values.data_ptr(),
                                                   cw_gu.meta.data_ptr(), out.data_ptr(), out.stride(0),
                                                   M, I, cw_gu.K, _dt(x), _stream())
-    _lib.check("sfb200_sparse_gemm_swiglu", rc)
+    if rc:
+        _lib.check("sfb200_sparse_gemm_swiglu", rc)
     return out
 
 
