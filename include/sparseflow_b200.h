@@ -87,6 +87,12 @@ SFB200_API int sfb200_prune_compress_24(const void* dense, int rows, int K, int 
                                         int tie, void* values, void* meta, void* ref_codes,
                                         void* pruned, void* stream);
 
+/* Compression of a weight that should be 2:4 already into the container of sfb200_blob_* (blob: device, 16-byte aligned,
+ * sfb200_blob_bytes(rows, K) bytes): header, values, padding and metadata in one pass.  *not_24_dev (device) becomes 1 if a
+ * group of four has more than two non-zeros, else 0.  K a multiple of 16, dense 16-byte aligned, ld a multiple of 8. */
+SFB200_API int sfb200_compress_blob_checked(const void* dense, int rows, int K, int ld, int dtype, int tie, void* blob,
+                                            int* not_24_dev, void* stream);
+
 /*
  * Same, for the fused gate|up weight of the gated FFN: reads gate[I, K] and up[I, K] and emits
  * the 2*I-row matrix whose rows alternate in blocks of 16 (16 gate rows, the matching 16 up

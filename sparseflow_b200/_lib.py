@@ -64,6 +64,7 @@ def lib() -> C.CDLL:
     L.sfb200_meta_bytes.argtypes = [i, i]
     L.sfb200_device_status.argtypes = [C.POINTER(C.c_int)]
     L.sfb200_prune_compress_24.argtypes = [vp, i, i, i, i, i, vp, vp, vp, vp, vp]
+    L.sfb200_compress_blob_checked.argtypes = [vp, i, i, i, i, i, vp, vp, vp]
     L.sfb200_prune_compress_gate_up.argtypes = [vp, vp, i, i, i, i, i, vp, vp, vp]
     L.sfb200_validate_24.argtypes = [vp, i, i, i, vp, vp]
     L.sfb200_decompress_24.argtypes = [vp, vp, i, i, vp, i, vp]

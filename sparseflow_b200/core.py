@@ -74,9 +74,10 @@ def compress_2_4(tensor: torch.Tensor) -> torch.Tensor:
     _require_lib()
     if tensor.dim() != 2:
         raise ValueError(f"expected a 2-D weight, got {tensor.dim()}-D")
-    if not validate_2_4(tensor):
+    blob, valid = serialize.compress_checked(tensor)
+    if not valid:
         raise ValueError("Tensor does not have valid 2:4 sparsity pattern")
-    return serialize.pack(ops.compress_weight(tensor))
+    return blob
 
 
 def sparse_mm(A: torch.Tensor, Bc: torch.Tensor, epilogue: str = "none",

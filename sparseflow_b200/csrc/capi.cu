@@ -144,6 +144,33 @@ int sfb200_prune_compress_24(const void* dense, int rows, int K, int ld, int dty
   return launch_prune_compress(a, static_cast<cudaStream_t>(stream));
 }
 
+int sfb200_compress_blob_checked(const void* dense, int rows, int K, int ld, int dtype, int tie, void* blob, int* not_24_dev,
+                                 void* stream) {
+  int err = kOk;
+  if (!device_state(&err)) return err;
+  if (dense == nullptr || blob == nullptr || not_24_dev == nullptr || (reinterpret_cast<uintptr_t>(blob) & 15)) return kErrInvalid;
+  unsigned char head[SFB200_BLOB_HEADER_BYTES];
+  const int rc = sfb200_blob_write_header(head, rows, K, dtype, tie == kTieLow ? SFB200_BLOB_TIE_LOW : 0u, 0);
+  if (rc != SFB200_SUCCESS) return rc;
+  Range r("sfb200.compress_blob_checked");
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
+  if (cudaMemsetAsync(not_24_dev, 0, sizeof(int), st) != cudaSuccess) return kErrCuda;
+  uint8_t* base = static_cast<uint8_t*>(blob);
+  PruneArgs a{};
+  a.dense = dense;
+  a.rows = rows;
+  a.K = K;
+  a.ld = ld;
+  a.fmt = dtype;
+  a.tie = tie;
+  a.values = base + SFB200_BLOB_HEADER_BYTES;
+  a.meta = base + sfb200_blob_bytes(rows, K) - meta_bytes(rows, K);
+  a.blob_head = head;
+  a.blob_dst = blob;
+  a.bad = not_24_dev;
+  return launch_prune_compress(a, st);
+}
+
 int sfb200_prune_compress_gate_up(const void* gate, const void* up, int I, int K, int ld, int dtype,
                                   int tie, void* values, void* meta, void* stream) {
   int err = kOk;

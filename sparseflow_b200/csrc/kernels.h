@@ -30,12 +30,16 @@ struct PruneArgs {
   int ld;
   int fmt;
   int tie;
-  int interleave;         // 0: out row r <- dense[r].  B>0 (needs dense2): blocks of B rows of
-                          // `dense` followed by the matching B rows of `dense2`; out rows = 2*rows
+  int interleave;         // 0: out row r <- dense[r].  16 (needs dense2): blocks of 16 rows of
+                          // `dense` followed by the matching 16 rows of `dense2`; out rows = 2*rows
   void* values;           // [out_rows, K/2]            or null
   void* meta;             // tiled metadata             or null
   void* ref_codes;        // [out_rows, K/4] uint8      or null
   void* pruned;           // [out_rows, K]              or null
+  // Checked compression into a container (csrc/blob.cpp), all or none; values and meta then lie inside the container.
+  const void* blob_head;  // HOST: the used 96 bytes of the header, written by the kernel
+  void* blob_dst;         // where the 256-byte header goes
+  int* bad;               // device, zeroed beforehand: set to 1 if a group of four has more than two non-zeros
 };
 int launch_prune_compress(const PruneArgs& a, cudaStream_t stream);
 // one int result: 1 if every group of four has <= 2 non-zeros

@@ -1,4 +1,4 @@
-// Launch of a GEMM kernel as a programmatic dependent of the kernel before it in the stream.
+// Launch of a kernel as a programmatic dependent of the kernel before it in the stream.
 //
 // The launch may begin while that kernel's last blocks still run: barriers, tensor memory and descriptors are set up and the
 // first weight tiles are prefetched into L2 under its tail, and every thread then executes griddepcontrol.wait
@@ -20,9 +20,9 @@ namespace sfb200 {
 
 // cluster = 0: as compiled (none, or __cluster_dims__).
 template <class... P, class... A>
-int launch_dependent(void (*kernel)(P...), int grid, int block, size_t smem, int cluster, cudaStream_t stream, A&&... args) {
+int launch_dependent(void (*kernel)(P...), dim3 grid, int block, size_t smem, int cluster, cudaStream_t stream, A&&... args) {
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(static_cast<unsigned>(grid), 1, 1);
+  cfg.gridDim = grid;
   cfg.blockDim = dim3(static_cast<unsigned>(block), 1, 1);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = stream;

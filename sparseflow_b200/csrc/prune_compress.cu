@@ -13,6 +13,10 @@
 //     lane = m0 + 8*kh + 16*m2, word = kb, bits [16*m1, 16*m1+16) = 4 nibbles (group j at 4j),
 //     nibble = idx0 | idx1 << 2.  Rows / K beyond the matrix are filled with nibble 0x4.
 //
+// Measured (B200, back to back): 11008 x 4096 24.0 us (5.87 TB/s), 28672 x 8192 111.6 us (6.58 TB/s), two 11008 x 4096 weights
+// interleaved 45.2 us (6.24 TB/s), two 28672 x 8192 220.6 us; before the interleave block was a constant and the launches
+// were programmatic dependents (launch.h) 26.7, 116.9, 53.2 and 255.2 us.
+//
 // HBM-bound: 2 B read + 1 B values + 1/8 B metadata per weight element.  One thread owns 16
 // consecutive K elements of rows m and m+8 (two 16-byte loads per row), which is exactly one
 // 32-bit metadata word; a warp streams 1 KiB of each of its two rows.
@@ -25,8 +29,11 @@
 // memory that returns the kept pair as a metadata nibble and as the byte selector that gathers the two kept values.
 #include <cuda_runtime.h>
 #include <stdint.h>
+#include <string.h>
 
 #include "kernels.h"
+#include "launch.h"
+#include "sm100_ptx.cuh"
 
 namespace sfb200 {
 namespace {
@@ -122,32 +129,57 @@ struct PruneParams {
   uint32_t clamp2;     // (inf pattern + 1) in both 16-bit halves
 };
 
+// Container header of a checked compression, written by the kernel (CHECK below).
+constexpr unsigned kBlobHeadWords = 64, kBlobHeadUsed = 24;
+struct BlobHead {
+  uint32_t words[kBlobHeadUsed];
+  uint32_t* dst;
+  uint8_t* pad;        // zero padding between values and metadata
+  int pad_bytes;       // < 256
+  int* bad;            // zeroed by the caller
+};
+
+// Source row of output row r.  Interleaved: 16 rows of src0, then the 16 matching rows of src1.  (The block of 16 is a
+// constant: with a run-time one its divisions were a quarter of the gate|up kernel's instructions.)
+constexpr int kInterleave = 16;
 __device__ __forceinline__ const uint16_t* src_row(const PruneParams& p, int r) {
-  if (p.interleave == 0) return p.src0 + static_cast<size_t>(r) * p.ld;
-  const int B = p.interleave;
-  const int blk = r / (2 * B), w = r % (2 * B);
-  const uint16_t* base = (w < B) ? p.src0 : p.src1;
-  return base + static_cast<size_t>(blk * B + (w % B)) * p.ld;
+  if (!p.interleave) return p.src0 + static_cast<size_t>(r) * p.ld;
+  const uint16_t* base = (r / kInterleave) & 1 ? p.src1 : p.src0;
+  return base + static_cast<size_t>(r / (2 * kInterleave) * kInterleave + r % kInterleave) * p.ld;
 }
 
-// Processes 16 elements of one row; returns the 16-bit metadata half word.
-template <int TIE>
-__device__ __forceinline__ uint32_t process_row16(const PruneParams& p, const uint32_t* lut, int r, int k0) {
-  if (r >= p.out_rows || k0 >= p.K) return kPadMeta16;
+// 16 consecutive elements of one row, as loaded.
+struct Row16 {
+  uint4 a, b;
+};
+__device__ __forceinline__ Row16 load_row16(const PruneParams& p, int r, int k0) {
   const uint4* s = reinterpret_cast<const uint4*>(src_row(p, r) + k0);
-  const uint4 a = __ldg(s), b = __ldg(s + 1);
+  return Row16{__ldg(s), __ldg(s + 1)};
+}
+
+// More than two non-zeros in a group of four (lo, hi), for either of two groups at once.
+__device__ __forceinline__ bool not_24(uint32_t lo0, uint32_t hi0, uint32_t lo1, uint32_t hi1) {
+  // element i of both groups side by side, 1 where its magnitude is not zero
+  const uint32_t n = min_u16x2(__byte_perm(lo0, lo1, 0x5410) & 0x7FFF7FFFu, 0x00010001u) +
+                     min_u16x2(__byte_perm(lo0, lo1, 0x7632) & 0x7FFF7FFFu, 0x00010001u) +
+                     min_u16x2(__byte_perm(hi0, hi1, 0x5410) & 0x7FFF7FFFu, 0x00010001u) +
+                     min_u16x2(__byte_perm(hi0, hi1, 0x7632) & 0x7FFF7FFFu, 0x00010001u);
+  return ((n + 0x00010001u) & 0x00040004u) != 0;     // count 3 or 4
+}
+
+// Prunes 16 consecutive elements and stores them at the outputs' own element offsets; returns their metadata half word.
+template <int TIE>
+__device__ __forceinline__ uint32_t prune_store16(const PruneParams& p, const uint32_t* lut, const uint4& a, const uint4& b,
+                                                  size_t at_values, size_t at_pruned, size_t at_codes) {
   uint32_t e0, e1, e2, e3;
   select_pair<TIE>(a.x, a.y, a.z, a.w, p.clamp2, lut, e0, e1);
   select_pair<TIE>(b.x, b.y, b.z, b.w, p.clamp2, lut, e2, e3);
   const bool want_pruned = p.pruned != nullptr;
   const GroupOut g0 = finish_group(a.x, a.y, e0, want_pruned), g1 = finish_group(a.z, a.w, e1, want_pruned);
   const GroupOut g2 = finish_group(b.x, b.y, e2, want_pruned), g3 = finish_group(b.z, b.w, e3, want_pruned);
-  if (p.values) {
-    uint4 v = make_uint4(g0.vals, g1.vals, g2.vals, g3.vals);
-    *reinterpret_cast<uint4*>(p.values + static_cast<size_t>(r) * (p.K / 2) + k0 / 2) = v;
-  }
+  if (p.values) *reinterpret_cast<uint4*>(p.values + at_values) = make_uint4(g0.vals, g1.vals, g2.vals, g3.vals);
   if (want_pruned) {
-    uint4* d = reinterpret_cast<uint4*>(p.pruned + static_cast<size_t>(r) * p.K + k0);
+    uint4* d = reinterpret_cast<uint4*>(p.pruned + at_pruned);
     d[0] = make_uint4(g0.lo, g0.hi, g1.lo, g1.hi);
     d[1] = make_uint4(g2.lo, g2.hi, g3.lo, g3.hi);
   }
@@ -156,33 +188,86 @@ __device__ __forceinline__ uint32_t process_row16(const PruneParams& p, const ui
                        static_cast<uint32_t>((kRefCodeLut >> (4 * g1.nib)) & 0xF) << 8 |
                        static_cast<uint32_t>((kRefCodeLut >> (4 * g2.nib)) & 0xF) << 16 |
                        static_cast<uint32_t>((kRefCodeLut >> (4 * g3.nib)) & 0xF) << 24;
-    *reinterpret_cast<uint32_t*>(p.ref_codes + static_cast<size_t>(r) * (p.K / 4) + k0 / 4) = c;
+    *reinterpret_cast<uint32_t*>(p.ref_codes + at_codes) = c;
   }
   return (e0 >> 16) | ((e1 >> 12) & 0xF0u) | ((e2 >> 8) & 0xF00u) | ((e3 >> 4) & 0xF000u);
 }
 
-// grid: (ceil(Kpad / 512), Rpad / 16), block 256: warp w -> rows m0 = w and w + 8 of the 16-row
-// group, lane -> 16-element K slice.
+// The same for one group of four.
 template <int TIE>
-__global__ void __launch_bounds__(256) prune_compress_kernel(const PruneParams p) {
+__device__ __forceinline__ void prune_store4(const PruneParams& p, const uint32_t* lut, const uint2& v, size_t e) {
+  uint32_t e0, e1;
+  select_pair<TIE>(v.x, v.y, v.x, v.y, p.clamp2, lut, e0, e1);
+  const GroupOut o = finish_group(v.x, v.y, e0, p.pruned != nullptr);
+  if (p.values) *reinterpret_cast<uint32_t*>(p.values + e / 2) = o.vals;
+  if (p.pruned) *reinterpret_cast<uint2*>(p.pruned + e) = make_uint2(o.lo, o.hi);
+  if (p.ref_codes) p.ref_codes[e / 4] = static_cast<uint8_t>((kRefCodeLut >> (4 * o.nib)) & 0xF);
+}
+
+// 16 elements of row r; returns the 16-bit metadata half word.  CHECK: sets `bad` if they are not 2:4.
+template <int TIE, bool CHECK>
+__device__ __forceinline__ uint32_t process_row16(const PruneParams& p, const uint32_t* lut, int r, int k0, bool& bad) {
+  if (r >= p.out_rows || k0 >= p.K) return kPadMeta16;
+  const Row16 w = load_row16(p, r, k0);
+  if (CHECK) bad |= not_24(w.a.x, w.a.y, w.a.z, w.a.w) || not_24(w.b.x, w.b.y, w.b.z, w.b.w);
+  return prune_store16<TIE>(p, lut, w.a, w.b, static_cast<size_t>(r) * (p.K / 2) + k0 / 2, static_cast<size_t>(r) * p.K + k0,
+                            static_cast<size_t>(r) * (p.K / 4) + k0 / 4);
+}
+
+// grid: (ceil(Kpad / 512), Rpad / 16), block 256: warp w -> rows m0 = w and w + 8 of the 16-row
+// group, lane -> 16-element K slice.  (Loading both rows before processing either, with and without streaming hints, measured
+// within 5 % either way: occupancy already covers the latency.)
+// CHECK: additionally sets *bad when a group of the source has more than two non-zeros (the weight is not 2:4), and the
+// first block writes the container header and the zero padding before the metadata.
+template <int TIE, bool CHECK>
+__global__ void __launch_bounds__(256, CHECK ? 6 : 8) prune_compress_kernel(const __grid_constant__ PruneParams p,
+                                                             const __grid_constant__ BlobHead head) {
   __shared__ uint32_t lut[64];
   if (threadIdx.x < 64) lut[threadIdx.x] = kSelectLut.e[threadIdx.x];
   __syncthreads();
+  dependency_wait();
+  dependency_trigger();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int k0 = (blockIdx.x * 32 + lane) * 16;
-  if (k0 >= p.k_tiles128 * 128) return;
   const int r_a = blockIdx.y * 16 + warp;
-  const uint32_t ma = process_row16<TIE>(p, lut, r_a, k0);
-  const uint32_t mb = process_row16<TIE>(p, lut, r_a + 8, k0);
+  if (CHECK && blockIdx.x == 0 && blockIdx.y == 0) {
+    if (threadIdx.x < kBlobHeadWords) head.dst[threadIdx.x] = threadIdx.x < kBlobHeadUsed ? head.words[threadIdx.x] : 0u;
+    if (static_cast<int>(threadIdx.x) < head.pad_bytes) head.pad[threadIdx.x] = 0;
+  }
+  if (k0 >= p.k_tiles128 * 128) return;
+  bool bad = false;
+  const uint32_t ma = process_row16<TIE, CHECK>(p, lut, r_a, k0, bad);
+  const uint32_t mb = process_row16<TIE, CHECK>(p, lut, r_a + 8, k0, bad);
   if (p.meta) {
     const int rt = r_a >> 7, m2 = (r_a & 127) >> 4;
     const int kt = k0 >> 7, kb = (k0 & 127) >> 5, kh = (k0 & 31) >> 4;
     const int ln = warp + 8 * kh + 16 * m2;
     p.meta[((static_cast<size_t>(rt) * p.k_tiles128 + kt) * 128 + ln) * 4 + kb] = ma | (mb << 16);
   }
+  if (CHECK && bad) *head.bad = 1;
 }
 
-// Any K % 4 == 0: one thread per group, no tiled metadata.
+// Any K % 4 == 0, rows without padding between them, no tiled metadata: without the tile layout a weight is one run of
+// n = rows * K elements, so a thread takes 16 of them whatever K is (the last one the groups that are left).
+template <int TIE>
+__global__ void __launch_bounds__(256) prune_flat_kernel(const __grid_constant__ PruneParams p, size_t n) {
+  __shared__ uint32_t lut[64];
+  if (threadIdx.x < 64) lut[threadIdx.x] = kSelectLut.e[threadIdx.x];
+  __syncthreads();
+  dependency_wait();
+  dependency_trigger();
+  const size_t e = (blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x) * 16;
+  if (e >= n) return;
+  const uint16_t* s = p.src0 + e;
+  if (e + 16 <= n) {
+    const uint4 a = __ldg(reinterpret_cast<const uint4*>(s)), b = __ldg(reinterpret_cast<const uint4*>(s) + 1);
+    prune_store16<TIE>(p, lut, a, b, e / 2, e, e / 4);
+  } else {
+    for (size_t i = e; i < n; i += 4) prune_store4<TIE>(p, lut, *reinterpret_cast<const uint2*>(p.src0 + i), i);
+  }
+}
+
+// Any K % 4 == 0 and row pitch: one thread per group, no tiled metadata.
 template <int TIE>
 __global__ void prune_generic_kernel(const PruneParams p) {
   __shared__ uint32_t lut[64];
@@ -193,15 +278,7 @@ __global__ void prune_generic_kernel(const PruneParams p) {
   for (size_t i = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x; i < total;
        i += static_cast<size_t>(gridDim.x) * blockDim.x) {
     const int r = static_cast<int>(i / G), g = static_cast<int>(i % G);
-    const uint2 v = *reinterpret_cast<const uint2*>(src_row(p, r) + 4 * g);
-    uint32_t e0, e1;
-    select_pair<TIE>(v.x, v.y, v.x, v.y, p.clamp2, lut, e0, e1);
-    const GroupOut o = finish_group(v.x, v.y, e0, p.pruned != nullptr);
-    if (p.values) *reinterpret_cast<uint32_t*>(p.values + static_cast<size_t>(r) * (p.K / 2) + 2 * g) = o.vals;
-    if (p.pruned)
-      *reinterpret_cast<uint2*>(p.pruned + static_cast<size_t>(r) * p.K + 4 * g) = make_uint2(o.lo, o.hi);
-    if (p.ref_codes)
-      p.ref_codes[static_cast<size_t>(r) * G + g] = static_cast<uint8_t>((kRefCodeLut >> (4 * o.nib)) & 0xF);
+    prune_store4<TIE>(p, lut, *reinterpret_cast<const uint2*>(src_row(p, r) + 4 * g), 4 * i);
   }
 }
 
@@ -216,6 +293,24 @@ __global__ void validate_24_kernel(const uint16_t* w, int rows, int K, int ld, i
     const int nz = ((v.x & 0x7FFF) != 0) + ((v.x & 0x7FFF0000) != 0) + ((v.y & 0x7FFF) != 0) +
                    ((v.y & 0x7FFF0000) != 0);
     bad |= nz > 2;
+  }
+  if (bad) atomicExch(flag, 0);
+}
+
+// The same over one run of n elements (rows without padding between them): 16 per thread and load round.
+__global__ void __launch_bounds__(256) validate_flat_kernel(const uint16_t* w, size_t n, int* flag) {
+  bool bad = false;
+  const size_t step = static_cast<size_t>(gridDim.x) * blockDim.x * 16;
+  for (size_t e = (blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x) * 16; e < n; e += step) {
+    if (e + 16 <= n) {
+      const uint4 a = __ldg(reinterpret_cast<const uint4*>(w + e)), b = __ldg(reinterpret_cast<const uint4*>(w + e) + 1);
+      bad |= not_24(a.x, a.y, a.z, a.w) || not_24(b.x, b.y, b.z, b.w);
+    } else {
+      for (size_t i = e; i < n; i += 4) {
+        const uint2 v = *reinterpret_cast<const uint2*>(w + i);
+        bad |= not_24(v.x, v.y, v.x, v.y);
+      }
+    }
   }
   if (bad) atomicExch(flag, 0);
 }
@@ -247,7 +342,7 @@ __global__ void decompress_kernel(const uint16_t* values, const uint32_t* meta, 
 int launch_prune_compress(const PruneArgs& a, cudaStream_t stream) {
   if (a.rows <= 0 || a.K <= 0 || a.K % 4 != 0 || a.dense == nullptr) return kErrInvalid;
   if (a.ld < a.K || a.ld % 4 != 0) return kErrInvalid;
-  if (a.interleave != 0 && (a.dense2 == nullptr || a.interleave < 0 || a.rows % a.interleave != 0))
+  if (a.interleave != 0 && (a.dense2 == nullptr || a.interleave != kInterleave || a.rows % kInterleave != 0))
     return kErrInvalid;
   if (a.fmt != kF16 && a.fmt != kBF16) return kErrInvalid;
   PruneParams p;
@@ -271,12 +366,34 @@ int launch_prune_compress(const PruneArgs& a, cudaStream_t stream) {
     const int kpad = p.k_tiles128 * 128;
     const int rpad = ((p.out_rows + 127) / 128) * 128;
     dim3 grid((kpad + 511) / 512, rpad / 16);
-    if (a.tie == kTieLow) prune_compress_kernel<kTieLow><<<grid, 256, 0, stream>>>(p);
-    else prune_compress_kernel<kTieHigh><<<grid, 256, 0, stream>>>(p);
+    BlobHead head = {};
+    if (a.blob_head != nullptr) {
+      memcpy(head.words, a.blob_head, sizeof(head.words));
+      head.dst = static_cast<uint32_t*>(a.blob_dst);
+      head.pad = static_cast<uint8_t*>(a.values) + values_bytes(p.out_rows, a.K);
+      head.pad_bytes = static_cast<int>(static_cast<uint8_t*>(a.meta) - head.pad);
+      head.bad = a.bad;
+      if (head.pad_bytes < 0 || head.pad_bytes >= 256) return kErrInvalid;
+      if (a.tie == kTieLow) return launch_dependent(prune_compress_kernel<kTieLow, true>, grid, 256, 0, 0, stream, p, head);
+      else return launch_dependent(prune_compress_kernel<kTieHigh, true>, grid, 256, 0, 0, stream, p, head);
+    } else if (a.tie == kTieLow) {
+      return launch_dependent(prune_compress_kernel<kTieLow, false>, grid, 256, 0, 0, stream, p, head);
+    } else {
+      return launch_dependent(prune_compress_kernel<kTieHigh, false>, grid, 256, 0, 0, stream, p, head);
+    }
   } else {
-    if (a.meta != nullptr) return kErrInvalid;  // tiled metadata needs K % 16 == 0 and 16-byte alignment
+    if (a.meta != nullptr || a.blob_head != nullptr) return kErrInvalid;  // tiled metadata needs K % 16 == 0 and 16-byte alignment
     if ((reinterpret_cast<uintptr_t>(a.dense) | reinterpret_cast<uintptr_t>(a.dense2)) % 8 != 0)
       return kErrInvalid;
+    // One run of elements, 16 per thread, where source and outputs allow 16-byte accesses: 4000 x 1012 8.5 -> 4.7 us.
+    if (a.ld == a.K && a.interleave == 0 &&
+        ((reinterpret_cast<uintptr_t>(a.dense) | reinterpret_cast<uintptr_t>(a.values) | reinterpret_cast<uintptr_t>(a.pruned) |
+          reinterpret_cast<uintptr_t>(a.ref_codes)) % 16 == 0)) {
+      const size_t n = static_cast<size_t>(a.rows) * a.K;
+      const dim3 grid(static_cast<unsigned>((n + 16 * 256 - 1) / (16 * 256)));
+      return a.tie == kTieLow ? launch_dependent(prune_flat_kernel<kTieLow>, grid, 256, 0, 0, stream, p, n)
+                              : launch_dependent(prune_flat_kernel<kTieHigh>, grid, 256, 0, 0, stream, p, n);
+    }
     const size_t total = static_cast<size_t>(p.out_rows) * (a.K / 4);
     const int blocks = static_cast<int>(total / 256 + 1 < 148 * 16 ? total / 256 + 1 : 148 * 16);
     if (a.tie == kTieLow) prune_generic_kernel<kTieLow><<<blocks, 256, 0, stream>>>(p);
@@ -288,6 +405,12 @@ int launch_prune_compress(const PruneArgs& a, cudaStream_t stream) {
 int launch_validate_24(const void* w, int rows, int K, int ld, int* d_flag, cudaStream_t stream) {
   if (rows <= 0 || K <= 0 || K % 4 != 0 || ld % 4 != 0 || (reinterpret_cast<uintptr_t>(w) % 8) != 0)
     return kErrInvalid;
+  if (ld == K && reinterpret_cast<uintptr_t>(w) % 16 == 0) {   // 11008 x 4096: 35.0 -> 22.3 us
+    const size_t n = static_cast<size_t>(rows) * K, need = (n + 16 * 256 - 1) / (16 * 256);
+    const int blocks = static_cast<int>(need < 148 * 8 ? need : 148 * 8);
+    validate_flat_kernel<<<blocks, 256, 0, stream>>>(static_cast<const uint16_t*>(w), n, d_flag);
+    return cudaGetLastError() == cudaSuccess ? kOk : kErrCuda;
+  }
   const size_t total = static_cast<size_t>(rows) * (K / 4);
   const int blocks = static_cast<int>(total / 256 + 1 < 148 * 16 ? total / 256 + 1 : 148 * 16);
   validate_24_kernel<<<blocks, 256, 0, stream>>>(static_cast<const uint16_t*>(w), rows, K, ld, d_flag);

@@ -66,6 +66,27 @@ def pack(cw: Compressed24, tie: str = "high", checksum: bool = False) -> torch.T
     return blob
 
 
+def compress_checked(w: torch.Tensor):
+    """(blob, valid) of a 2-D weight: its packed form and whether it is 2:4 already.  One kernel reads the weight once,
+    checks it and writes header, values and metadata in place; what that kernel does not take (a width that is no
+    multiple of 16, an unaligned view, another type) goes through the separate check, compression and packing."""
+    from . import ops
+    if (w.is_cuda and w.dim() == 2 and w.dtype in _DT and w.numel() > 0 and w.shape[1] % 16 == 0):
+        src = w if w.stride(1) == 1 else w.contiguous()
+        if src.data_ptr() % 16 == 0 and src.stride(0) % 8 == 0 and src.stride(0) >= src.shape[1]:
+            rows, K = src.shape
+            with ops._on(src.device):
+                blob = torch.empty(blob_bytes(rows, K), dtype=torch.uint8, device=src.device)
+                flag = torch.empty(1, dtype=torch.int32, device=src.device)
+                rc = _lib.lib().sfb200_compress_blob_checked(src.data_ptr(), rows, K, src.stride(0), _DT[src.dtype],
+                                                             ops.TIE_HIGH, blob.data_ptr(), flag.data_ptr(), ops._stream())
+            _lib.check("sfb200_compress_blob_checked", rc)
+            return blob, flag.item() == 0
+    if not ops.validate_24(w):
+        return None, False
+    return pack(ops.compress_weight(w)), True
+
+
 def unpack(blob: torch.Tensor, verify_checksum: bool = False) -> Compressed24:
     """Views of the values and the metadata inside ``blob``.  Raises on a foreign, truncated or
     corrupt blob and on a layout version this library does not read."""
