@@ -138,6 +138,9 @@ int route_sparse_gemm(int m_tok, int n_out, int K, int epi, int num_sms);
 // ---- small-M (decode) sparse GEMM ----------------------------------------------------------
 // Supports M <= 32 tokens; chosen by launch_sparse_gemm for m_tok <= kSmallMMaxTokens (force_bn == 8 forces it).
 int launch_sparse_gemm_small_m(const SparseGemmArgs& a, cudaStream_t stream);
+// Where the split-K cluster kernel applies too (few row tiles): whether this one is the faster, i.e. it has no second, partly
+// filled round of 16-row slabs -- at most one slab per SM, or two blocks per SM with the X cache in shared memory.
+bool small_m_beats_splitk(int m_tok, int n_out, int K, int num_sms);
 constexpr int kSmallMMaxTokens = 4;   // from 5 tokens the tcgen05 kernel with a 32-token tile is faster (measured)
 
 // ---- elementwise -----------------------------------------------------------------------------

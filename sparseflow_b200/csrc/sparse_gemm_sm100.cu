@@ -452,6 +452,13 @@ int route_sparse_gemm(int m_tok, int n_out, int K, int epi, int num_sms) {
   const int fixed = plan_sparse_gemm(m_tok, n_out, K, epi, num_sms);
   if (m_tok >= kPairMinTokens && fixed >= 1192 && fixed <= 1240)
     return pick_pair_variant_sustained(n_out, m_tok, K, num_sms, epi == kEpiSwiGLU);
+  if (m_tok <= 8 && epi == kEpiStore) {
+    // decode on few row tiles: slab kernel or split K.  Measured at 1 / 2 / 8 tokens, slabs against split K: 2048 x 2048 2.8 /
+    // 3.0 / 4.0 against 4.5 us; 4096 x 4096 5.3 / 6.0 / 8.4 against 6.8-7.2; 4096 x 11008 11.0 / 13.6 / 20.1 against 11.8;
+    // 4096 x 14336 15.3 / 16.6 / 24.9 against 13.9; 8192 x 8192 15.3 / 17.0 / 21.8 against 15.8.
+    const int split = splitk_factor(m_tok, n_out, K, num_sms);
+    if (split > 1) return small_m_beats_splitk(m_tok, n_out, K, num_sms) ? 8 : (split == 4 ? 4000 : 3000) + splitk_token_tile(m_tok);
+  }
   if (m_tok <= 64 || m_tok >= kPairMinTokens) return fixed;
   double band_us = 0.0, fixed_us = 0.0;
   const int band = pick_band_variant(m_tok, n_out, K, num_sms, &band_us);

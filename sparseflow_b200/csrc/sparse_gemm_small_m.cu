@@ -18,7 +18,12 @@
 //     cp.async ring as the values, so no MMA waits on a DRAM-latency load;
 //   * X is tiny and every slab re-reads the same K slice per warp: each warp keeps its slice in
 //     shared memory already in B-fragment order (one 16-byte read per k-step and 8 tokens) when it
-//     fits, else reads it through L1.
+//     fits, else reads it through L1.  It is filled after the first weight copies have been issued, with 16-byte loads:
+//     filled before them, one 4-byte load per lane and fragment word, it put 2-3 us of L2 latency in front of every call.
+//
+// Measured (B200, back to back): one token 22016 x 4096 19.6 -> 18.9 us, 4096 x 11008 13.4 -> 11.0 us (4.6 TB/s), 4096 x 4096
+// 7.4 -> 5.3 us, 8192 x 8192 18.6 -> 15.3 us, 2048 x 2048 4.4 -> 2.8 us with the X cache filled behind the first weight
+// copies and the launch a programmatic dependent (launch.h).
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
@@ -125,27 +130,6 @@ __global__ void __launch_bounds__(kWarps * 32) sparse_gemm_small_m_kernel(const 
   dependency_wait();
   dependency_trigger();
 
-  // X fragment cache of this warp's K slice: xs[(k-step * NT + n) * 32 + lane] = (b0, b1, b2, b3)
-  uint4* xs = nullptr;
-  if (p.xs_ksteps > 0) {
-    uint8_t* xs_base = smem + kWarps * kWarpBytes + 2 * kWarps * kRows * 8 * NT * 4;
-    xs = reinterpret_cast<uint4*>(xs_base) + static_cast<size_t>(warp) * p.xs_ksteps * NT * 32;
-    for (int ks = 0; ks < n_kt * 4; ++ks) {
-      const int k0 = (kt_lo * 4 + ks) * 32;
-#pragma unroll
-      for (int n = 0; n < NT; ++n) {
-        const int tok = n * 8 + g;
-        uint4 bv = make_uint4(0u, 0u, 0u, 0u);
-        if (tok < p.m_tok && k0 < p.K) {
-          const uint32_t* xp = reinterpret_cast<const uint32_t*>(p.x + static_cast<size_t>(tok) * p.ldx + k0 + 2 * t);
-          bv = make_uint4(__ldg(xp), __ldg(xp + 4), __ldg(xp + 8), __ldg(xp + 12));
-        }
-        xs[(ks * NT + n) * 32 + lane] = bv;
-      }
-    }
-    __syncwarp();
-  }
-
   // The cp.async ring runs continuously over this warp's (slab, k-tile) items, so the loads of the
   // next slab are in flight while the current one is reduced.
   const int my_slabs = (p.num_slabs - static_cast<int>(blockIdx.x) + static_cast<int>(gridDim.x) - 1) /
@@ -183,6 +167,34 @@ __global__ void __launch_bounds__(kWarps * 32) sparse_gemm_small_m_kernel(const 
   };
 #pragma unroll
   for (int i = 0; i < kStages - 1; ++i) issue_next();
+
+  // X fragment cache of this warp's K slice, filled while the first weights are on their way:
+  // xs[(k-step * m_tok + token) * 4 + t] = (b0, b1, b2, b3) of lane (g = token % 8, t).  16 contiguous bytes of a token are
+  // word q of four neighbouring lanes' fragments.  Tokens beyond m_tok have no entries: their lanes read the last token's,
+  // and the columns they produce are not stored.
+  uint4* xs = nullptr;
+  if (p.xs_ksteps > 0) {
+    uint8_t* xs_base = smem + kWarps * kWarpBytes + 2 * kWarps * kRows * 8 * NT * 4;
+    xs = reinterpret_cast<uint4*>(xs_base) + static_cast<size_t>(warp) * p.xs_ksteps * p.m_tok * 4;
+    const int k_lo = kt_lo * 128, k_hi = kt_hi * 128 < p.K ? kt_hi * 128 : p.K;
+    const int chunks = k_hi > k_lo ? (k_hi - k_lo) / 8 : 0;      // K % 64 == 0: whole 16-byte chunks
+#pragma unroll 4
+    for (int i = lane; i < chunks * p.m_tok; i += 32) {
+      const int tok = i / chunks, c = i - tok * chunks;
+      const uint4 v = __ldg(reinterpret_cast<const uint4*>(p.x + static_cast<size_t>(tok) * p.ldx + k_lo + c * 8));
+      uint32_t* d = reinterpret_cast<uint32_t*>(xs + ((c >> 2) * p.m_tok + tok) * 4) + (c & 3);
+      d[0] = v.x;
+      d[4] = v.y;
+      d[8] = v.z;
+      d[12] = v.w;
+    }
+    // K steps of the last tile beyond K: their weights are zero-filled, and zero times whatever lay here must be zero
+    for (int i = chunks / 4 * p.m_tok * 4 + lane; i < n_kt * 4 * p.m_tok * 4; i += 32) xs[i] = make_uint4(0u, 0u, 0u, 0u);
+    __syncwarp();
+  }
+  int xs_at[NT];
+#pragma unroll
+  for (int n = 0; n < NT; ++n) xs_at[n] = (n * 8 + g < p.m_tok ? n * 8 + g : p.m_tok - 1) * 4 + t;
 
   // L1 path for X (used when the fragment cache does not fit): fragments of one k-tile
   uint32_t bnext[4][NT][4];
@@ -236,7 +248,7 @@ __global__ void __launch_bounds__(kWarps * 32) sparse_gemm_small_m_kernel(const 
 #pragma unroll
         for (int n = 0; n < NT; ++n) {
           if (xs != nullptr) {
-            const uint4 bv = xs[((i * 4 + kb) * NT + n) * 32 + lane];
+            const uint4 bv = xs[(i * 4 + kb) * p.m_tok * 4 + xs_at[n]];
             bcur[kb][n][0] = bv.x; bcur[kb][n][1] = bv.y; bcur[kb][n][2] = bv.z; bcur[kb][n][3] = bv.w;
           } else {
 #pragma unroll
@@ -308,15 +320,19 @@ __global__ void __launch_bounds__(kWarps * 32) sparse_gemm_small_m_kernel(const 
   cp_async_wait<0>();
 }
 
+// Shared memory: weight ring, two reduction buffers and, if it leaves room, the X fragment cache (64 B per k-step and
+// token; *ksteps = k-steps per warp it holds, 0 = none).
+constexpr int kTwoCtaSmem = 110 * 1024;
+int small_m_smem(int sl, int nt, int m_tok, int k_tiles128, int* ksteps) {
+  const int smem = kWarps * kWarpSmemFor(sl) + 2 * kWarps * 16 * sl * 8 * nt * 4;
+  const int steps = ((k_tiles128 + kWarps - 1) / kWarps) * 4, xs_bytes = kWarps * steps * m_tok * 64;
+  *ksteps = smem + xs_bytes <= 226 * 1024 ? steps : 0;
+  return *ksteps ? smem + xs_bytes : smem;
+}
+
 template <int NT, int SL, bool SWIGLU, bool BF16>
 int launch_nt(SmallParams p, int num_sms, cudaStream_t stream) {
-  int smem = kWarps * kWarpSmemFor(SL) + 2 * kWarps * 16 * SL * 8 * NT * 4;
-  {  // X fragment cache if it leaves room (k-steps per warp x NT x 512 B x 8 warps)
-    const int ksteps = ((p.k_tiles128 + kWarps - 1) / kWarps) * 4;
-    const int xs_bytes = kWarps * ksteps * NT * 512;
-    p.xs_ksteps = (smem + xs_bytes <= 200 * 1024) ? ksteps : 0;
-    if (p.xs_ksteps) smem += xs_bytes;
-  }
+  const int smem = small_m_smem(SL, NT, p.m_tok, p.k_tiles128, &p.xs_ksteps);
   static bool attr_set[16] = {};
   int dev = 0;
   cudaGetDevice(&dev);
@@ -329,7 +345,7 @@ int launch_nt(SmallParams p, int num_sms, cudaStream_t stream) {
   // resident CTAs per SM: the count (1 or 2) that needs the fewest bandwidth-rounds
   const long units = p.num_slabs;
   const long r1 = (units + num_sms - 1) / num_sms, r2 = (units + 2L * num_sms - 1) / (2L * num_sms);
-  const bool two = smem <= 110 * 1024 && 2 * r2 <= r1;
+  const bool two = smem <= kTwoCtaSmem && 2 * r2 <= r1;
   long ctas = static_cast<long>(num_sms) * (two ? 2 : 1);
   if (ctas > units) ctas = units;
   return launch_dependent(sparse_gemm_small_m_kernel<NT, SL, SWIGLU, BF16>, static_cast<int>(ctas), kWarps * 32, smem, 0, stream, p);
@@ -347,9 +363,17 @@ int dispatch_nt(const SmallParams& p, int nt, bool bf, int num_sms, cudaStream_t
 
 }  // namespace
 
+bool small_m_beats_splitk(int m_tok, int n_out, int K, int num_sms) {
+  if (m_tok > 8 || m_tok * ((K + 127) / 128) > 192) return false;   // (1536 x 4096 at 8 tokens: 6.3 against 5.7 us)
+  const int units = (n_out + 15) / 16;
+  int ksteps = 0;
+  const int smem = small_m_smem(1, 1, m_tok, (K + 127) / 128, &ksteps);
+  return ksteps > 0 && (units <= num_sms || (smem <= kTwoCtaSmem && units <= 4 * num_sms));
+}
+
 int launch_sparse_gemm_small_m(const SparseGemmArgs& a, cudaStream_t stream) {
   if (a.m_tok <= 0 || a.m_tok > 8 * kMaxNT || a.K % 64 != 0 || a.n_out <= 0) return kErrInvalid;
-  if (a.ldx % 2 != 0 || (reinterpret_cast<uintptr_t>(a.x) & 3) || (reinterpret_cast<uintptr_t>(a.values) & 15) ||
+  if (a.ldx % 8 != 0 || (reinterpret_cast<uintptr_t>(a.x) & 15) || (reinterpret_cast<uintptr_t>(a.values) & 15) ||
       (reinterpret_cast<uintptr_t>(a.meta) & 15) || (a.K / 2) % 8 != 0)
     return kErrInvalid;
   if (a.epi == kEpiSwiGLU && a.n_out % 32 != 0) return kErrInvalid;

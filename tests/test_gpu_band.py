@@ -15,16 +15,18 @@ def _route(M, N, K, sw=0, sms=148):
 
 def test_route_takes_known_forms():
     """Band forms only from 65 to 1023 tokens, with a legal tile; from 1024 tokens a 256-row pair tile may give way to a
-    512-row one; everything else is the fixed-tile plan."""
+    512-row one; up to 8 tokens on few row tiles the slab kernel and split K may swap; everything else is the plan."""
     plan = _lib.lib().sfb200_debug_plan_gemm
     for sms in (148, 132, 64, 2):
         for N, K in ((4096, 4096), (22016, 4096), (4096, 11008), (57344, 8192), (8, 64), (392, 1088), (1024, 512)):
-            for M in (1, 32, 64, 65, 100, 160, 161, 256, 257, 300, 512, 777, 1023, 1024, 5000):
+            for M in (1, 2, 5, 8, 32, 64, 65, 100, 160, 161, 256, 257, 300, 512, 777, 1023, 1024, 5000):
                 v = _route(M, N, K, 0, sms)
                 if v >= 6000:
                     t = v % 1000
                     assert 64 < M < 1024 and v < 8000 and 16 <= t <= 256 and t % 16 == 0, (M, N, K, sms, v)
                     assert v < 7000 or K >= 1024 - 127, (M, N, K, sms, v)
+                elif M <= 8 and v != plan(M, N, K, 0, sms):
+                    assert v in (8, 3032, 4032) and plan(M, N, K, 0, sms) in (8, 3032, 4032), (M, N, K, sms, v)
                 elif M >= 1024 and 1192 <= plan(M, N, K, 0, sms) <= 1240:
                     assert v in (1192, 1208, 1224, 1240, 5192, 5208, 5224, 5240), (M, N, K, sms, v)
                 else:
