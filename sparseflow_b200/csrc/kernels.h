@@ -131,6 +131,8 @@ int splitk_token_tile(int m_tok);
 int launch_sparse_gemm_band(const SparseGemmArgs& a, cudaStream_t stream);
 // The form of that kernel estimated fastest for a shape (6000 + t or 7000 + t) and its estimated time in us.
 int pick_band_variant(int m_tok, int n_out, int K, int num_sms, double* cost_us = nullptr);
+// Whether a split-1 form cuts left-over tiles into token slices for a shape.
+bool band_has_slices(int m_tok, int n_out, int num_sms, int variant);
 // What launch_sparse_gemm runs for a 16-bit result when nothing is forced: the band form where it is the faster one, a
 // 512-row pair tile where that needs less energy, else plan_sparse_gemm's choice among the fixed tiles.  Host-only.
 int route_sparse_gemm(int m_tok, int n_out, int K, int epi, int num_sms);

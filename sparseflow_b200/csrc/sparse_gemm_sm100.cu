@@ -441,13 +441,23 @@ int plan_sparse_gemm(int m_tok, int n_out, int K, int epi, int num_sms) {
   return pick_mid_variant(n_out, m_tok, K, num_sms, epi == kEpiSwiGLU);
 }
 
-// From 65 to 1023 tokens the band kernel (sparse_gemm_sm100_band.cu) is weighed against the fixed tiles.  Up to 160 tokens
-// it is taken outright: measured on 22016, 28672, 11008, 57344 x 4096 / 8192 and 4096, 8192, 2048-row weights it is 1.0-1.9 x
-// the fixed choice there (4096 x 11008 at 150 tokens 34.6 -> 18.5 us, 22016 x 4096 at 150 tokens 32.8 -> 27.1 us, 4096 x 4096
-// at 100 tokens 11.4 -> 11.3 us); above, the lower estimate decides (300 tokens: 34.4 -> 22.9 and 42.1 -> 34.8 us; 512
-// tokens: 34.9 -> 28.1 and 52.7 -> 47.1 us; at 700 tokens the two meet).  At 64 tokens and below a stage of the single-CTA
-// kernels carries as few token bytes as a pair's and their split-K form uses 128 SMs: 13.8 against 16.1 us on 4096 x 11008
-// at 24 tokens.
+// Estimated time in us of the single-CTA 64-token tiles: a 128-wide K step costs 0.215 us, the weights stream at 6.6 TB/s and
+// a third of the shorter of the two adds (11008 x 4096 at 64 tokens 13.5 us, 6000 x 3072 at 72 tokens 8.7 us, 8192 x 8192 at 128
+// tokens 22.0 us measured).
+double tile64_cost(int m_tok, int n_out, int K, int num_sms) {
+  const int tiles = ((n_out + 127) / 128) * ((m_tok + 63) / 64);
+  const double comp = ((tiles + num_sms - 1) / num_sms) * ((K + 127) / 128) * 0.215, hbm = n_out * (K * 1.125) / 6.6e6;
+  return 3.6 + (comp > hbm ? comp + hbm / 3.0 : hbm + comp / 3.0);
+}
+
+// From 33 to 1023 tokens the band kernel (sparse_gemm_sm100_band.cu) is weighed against the fixed tiles by estimated time.
+//   33-64 tokens: only where the plan would split K in two (38-74 row tiles): 8192 x 8192 at 64 tokens 20.8 -> 17.8 us, 6000 x
+//     3072 12.6 -> 9.1 us (the 64-token tile);
+//   65-128: against the 64-token tiles (6000 x 3072 at 72 tokens 8.7 against 10.1 us, 22016 x 4096 29.2 against 26.2);
+//   129-160: the band kernel outright, 1.1-1.9 x the fixed choice on every shape measured (4096 x 11008 at 150 tokens 34.6 ->
+//     18.5 us, 22016 x 4096 32.8 -> 25.2 us);
+//   above: the lower estimate (300 tokens: 4096 x 11008 34.4 -> 21.6 us, 22016 x 4096 42.1 -> 34.8 us; 520 tokens: 8192 x 8192
+//     55.5 -> 42.0 us; at 700-1000 tokens the two meet).
 int route_sparse_gemm(int m_tok, int n_out, int K, int epi, int num_sms) {
   const int fixed = plan_sparse_gemm(m_tok, n_out, K, epi, num_sms);
   if (m_tok >= kPairMinTokens && fixed >= 1192 && fixed <= 1240)
@@ -459,12 +469,17 @@ int route_sparse_gemm(int m_tok, int n_out, int K, int epi, int num_sms) {
     const int split = splitk_factor(m_tok, n_out, K, num_sms);
     if (split > 1) return small_m_beats_splitk(m_tok, n_out, K, num_sms) ? 8 : (split == 4 ? 4000 : 3000) + splitk_token_tile(m_tok);
   }
-  if (m_tok <= 64 || m_tok >= kPairMinTokens) return fixed;
+  if (m_tok >= kPairMinTokens || m_tok <= 32 || (m_tok <= 64 && (fixed < 3000 || fixed >= 4000))) return fixed;
   double band_us = 0.0, fixed_us = 0.0;
   const int band = pick_band_variant(m_tok, n_out, K, num_sms, &band_us);
+  if (m_tok <= 128) return tile64_cost(m_tok, n_out, K, num_sms) < band_us ? 64 : band;
   if (m_tok <= 160) return band;
   pick_mid_variant(n_out, m_tok, K, num_sms, epi == kEpiSwiGLU, &fixed_us);
-  return band_us < fixed_us ? band : fixed;
+  // The same tile as the fixed kernel's, with no left-over tiles to slice, has nothing to gain (2-4 % slower).  Above 800
+  // tokens the estimate is trusted by a wider margin: there the tiles with a single accumulator set fall behind it
+  // (8192 x 28672 at 1000 tokens estimated 0.95, measured 1.17 of the fixed tile).
+  if (band % 1000 == fixed % 1000 && fixed >= 1000 && fixed < 3000 && !band_has_slices(m_tok, n_out, num_sms, band)) return fixed;
+  return band_us < (m_tok > 800 ? 0.8 : 1.0) * fixed_us ? band : fixed;
 }
 
 int launch_sparse_gemm(const SparseGemmArgs& a, cudaStream_t stream) {

@@ -7,20 +7,23 @@
 // = 0.145 us + 1.02 ns * T for T tokens (the pair tiles of 192 ... 256 tokens measure 0.159 us + 1.02 ns * T).  A single
 // CTA would read every token column itself, twice that per column.  So below prefill the time of a GEMM is
 // (K steps in series) x (that step), and what is to be won is fewer steps in series with all pairs at work:
-//   * the token tile is a run-time multiple of 16 up to 256 (the ring gets as many stages as fit), so a tile is not wider
-//     than the tokens there are;
+//   * the token tile is a run-time multiple of 16 (the ring gets as many stages as fit), so a tile is not wider
+//     than the tokens there are.  Above 256 and up to 400 tokens it is two MMAs over one weight tile: 18 KB less to write per
+//     step than two tiles, a quarter less L2 traffic, and less energy, which is what counts at the power limit;
 //   * split 1: persistent pairs.  Tiles that fill whole passes over the pairs run at full width; those left over (fewer
-//     than pairs) are cut into token slices, as many as the idle pairs allow, so the last pass is short;
+//     than pairs) are cut into token slices, as many as the idle pairs allow, so the last pass is short.  A slice packs as
+//     many K steps into a ring stage as a whole tile's stage has room for: with one, the three stages of a 304-token
+//     ring kept 78 KB of a slice in flight and its step took 0.4 us of latency (22016 x 4096 at 300 tokens 40.3 us, now 36.9);
 //   * split 2 or 4 (few row tiles): a cluster of 2 or 4 pairs shares one tile, each pair streaming a slice of K.  The fp32
 //     accumulators are summed through distributed shared memory: pair p owns the 16-token chunks c with c % split == p,
 //     the others store theirs into its shared memory (the drained operand ring) as register fragments, 512 contiguous
 //     bytes per store instruction, and the owner adds them in pair order.  No scratch in global memory, no
 //     atomics, the same bits on every run.
 //
-// Measured (B200, CUDA-graph launches over weights that do not fit L2): 4096 x 11008 at 150 / 300 / 512 tokens 34.6 / 34.4 /
-// 34.9 -> 18.5 / 22.9 / 28.1 us, 22016 x 4096 (SiLU.mul) 32.8 / 42.1 / 52.7 -> 27.1 / 34.8 / 47.1 us, 4096 x 4096 at 300 tokens
-// 16.1 -> 12.7 us; evict-last token loads and evict-first stores are 3-10 % of that.  About 4 us of each launch are fixed:
-// 1.5 us to the first barrier, 1.6 us to the first operands, 0.9 us teardown; the exchange of split 2 costs 3.8 us at t = 160.
+// Measured (B200, steady load at the power limit, fixed tiles before -> now): 4096 x 11008 at 150 / 300 / 400 tokens 34.2 / 34.2 /
+// 36.2 -> 18.5 / 24.3 / 28.0 us; 22016 x 4096 (SiLU.mul) at 72 / 150 / 300 / 400 tokens 27.9 / 33.1 / 47.8 / 49.1 -> 25.5 / 28.3 /
+// 36.9 / 44.5 us; 8192 x 8192 at 520 tokens 55.5 -> 42.0 us; 57344 x 8192 at 300 tokens 219.7 -> 176.8 us.  Evict-last token loads and
+// evict-first stores are 3-10 % of that.  Split 4 and slices first measured slower (below).
 //
 // Warps: warp 0 = TMA producer, warp 1 = MMA issuer / tensor-memory owner, warps 2 ... 17 = epilogue.
 // All loads are plain per-CTA TMA copies.
@@ -53,7 +56,8 @@ __host__ __device__ constexpr int stage_bytes(int t) { return kABytes + kEBytes 
 __host__ __device__ constexpr int ring_stages(int t) {
   return kRingBytes / stage_bytes(t) < kMaxStages ? kRingBytes / stage_bytes(t) : kMaxStages;
 }
-static_assert(ring_stages(256) >= 4, "the widest tile keeps four stages");
+constexpr int kMaxTile = 400;
+static_assert(ring_stages(256) >= 4 && ring_stages(kMaxTile) >= 3, "the widest tiles keep three stages");
 static_assert(8 * (2 * kMaxStages + 4) + 16 <= kBarBytes, "barrier area");
 
 struct BandParams {
@@ -64,6 +68,9 @@ struct BandParams {
   int k_tiles128;
   int split;              // pairs per cluster = K slices
   int t_full, t_tail;     // tokens of a full item / of a slice of a left-over tile
+  int n0_full;            // columns of a full item's first MMA (the rest, if any, is a second one over the same weights)
+  int ks_tail;            // K steps per ring stage of a slice: what fits the stage of a full item
+  int tail_col;           // > 0: slices accumulate in columns of their own, from this one on
   int num_n_blks;         // token blocks of t_full
   int n_full;             // items [0, n_full) are whole tiles, the rest slices of the tiles from n_full on
   int slices;             // slices per left-over tile
@@ -74,6 +81,8 @@ struct BandParams {
 
 struct Item {
   int m_blk, tok0, tok_end, n;
+  int n0;         // columns [0, n0) and [n0, n) are one MMA each
+  int ks;         // K steps per ring stage
   bool tail;
 };
 // The i-th item of cluster c: whole tiles c, c + clusters, ..., then at most one slice of a left-over tile, slice c.
@@ -88,16 +97,35 @@ __device__ __forceinline__ bool get_item(int i, int c, int clusters, const BandP
   int tile = c + i * clusters, off = 0;
   it.tail = tile >= p.n_full;
   it.n = p.t_full;
+  it.n0 = p.n0_full;
+  it.ks = 1;
   if (it.tail) {
     tile = p.n_full + c / p.slices;
     off = (c % p.slices) * p.t_tail;
-    it.n = p.t_tail;
+    it.n = it.n0 = p.t_tail;
+    it.ks = p.ks_tail;
   }
   it.m_blk = tile / p.num_n_blks;
   const int t0 = (tile - it.m_blk * p.num_n_blks) * p.t_full;
   it.tok0 = t0 + off;
   it.tok_end = t0 + p.t_full < p.m_tok ? t0 + p.t_full : p.m_tok;
   return it.tok0 < it.tok_end;
+}
+
+// Accumulator of the next item: barrier index, its use count so far and first column.  `done` counts the items before it that
+// use the common set(s).
+__device__ __forceinline__ void next_acc(const BandParams& p, const Item& it, uint32_t& done, uint32_t& as, uint32_t& use,
+                                         uint32_t& col) {
+  if (it.tail && p.tail_col > 0) {      // at most one per pair
+    as = 1;
+    use = 0;
+    col = p.tail_col;
+    return;
+  }
+  as = p.acc_bufs == 2 ? (done & 1u) : 0u;
+  use = p.acc_bufs == 2 ? (done >> 1) : done;
+  col = as * p.t_full;
+  ++done;
 }
 
 __device__ __forceinline__ void st_cluster_v4(uint32_t addr, const uint32_t* r) {
@@ -114,14 +142,14 @@ __device__ __forceinline__ void add_f32(uint32_t& a, uint32_t b) { a = __float_a
 template <int EPI>
 __global__ void __launch_bounds__(kThreads, 1)
 sparse_gemm_band_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
-                        const __grid_constant__ CUtensorMap tmBt, const __grid_constant__ CUtensorMap tmE,
+                        const __grid_constant__ CUtensorMap tmB1, const __grid_constant__ CUtensorMap tmBt,
+                        const __grid_constant__ CUtensorMap tmE,
                         const BandParams p) {
   extern __shared__ uint8_t smem_raw[];
   // the same offset in every CTA of the cluster: the dynamic shared memory base is identical
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
   const uint32_t sbase = smem_u32(smem);
   const uint32_t st_bytes = static_cast<uint32_t>(stage_bytes(p.t_full));
-  const uint32_t off_e = kABytes + 128u * p.t_full;             // metadata within a stage
   const uint32_t staging = sbase + p.stages * st_bytes;
   const uint32_t bar_full = staging + kEpiWarps * kStagingBytes;   // used in the even CTA of the pair only
   const uint32_t bar_empty = bar_full + 8 * kMaxStages;            // both CTAs
@@ -158,7 +186,8 @@ sparse_gemm_band_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_co
     }
     mbar_fence_init();
     tma_prefetch_desc(&tmB);
-    tma_prefetch_desc(&tmBt);
+    if (p.n0_full < p.t_full) tma_prefetch_desc(&tmB1);
+    if (p.n_tail > 0) tma_prefetch_desc(&tmBt);
   }
   if (threadIdx.x == 64) {      // the first ring of weight tiles into L2, under the previous kernel's tail
     Item it;
@@ -194,21 +223,30 @@ sparse_gemm_band_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_co
         Item it;
         if (!get_item(i, cluster_id, num_clusters, p, it)) continue;
         const CUtensorMap* tb = it.tail ? &tmBt : &tmB;
-        const uint32_t b_sub = 64u * it.n;                       // bytes of one 64-wide K half of this CTA's tokens
+        const int n1 = it.n - it.n0;
+        const uint32_t b0 = 64u * it.n0, b1 = 64u * n1;          // bytes of one 64-wide K half of this CTA's tokens
         const int row0 = it.m_blk * 256 + static_cast<int>(rank) * 128;
-        const int tok = it.tok0 + static_cast<int>(rank) * (it.n / 2);
+        const int tok = it.tok0 + static_cast<int>(rank) * (it.n0 / 2), tok1 = it.tok0 + it.n0 + static_cast<int>(rank) * (n1 / 2);
         const int e_row = (row0 >> 7) * p.k_tiles128;
-        const uint32_t tx = 2u * (kABytes + kEBytes + 2u * b_sub);   // bytes of BOTH CTAs land on the even CTA's barrier
-        for (int kt = k_begin; kt < k_end; ++kt) {
+        const uint32_t step = stage_bytes(it.n);                 // weights, tokens, metadata of one K step
+        const uint32_t tx = 2u * (kABytes + kEBytes + 2u * (b0 + b1));   // bytes of BOTH CTAs land on the even CTA's barrier
+        for (int kt = k_begin; kt < k_end; kt += it.ks) {
           ok = mbar_wait(bar_empty + 8 * s, ph ^ 1, err, p.status, 1);
           if (!ok) break;
           const uint32_t full = pair_full0 + 8 * s;
-          const uint32_t st = sbase + s * st_bytes;
-          if (leader) mbar_arrive_expect_tx(bar_full + 8 * s, tx);
-          tma_load_2d_pair(st, &tmA, kt * 64, row0, full);
-          tma_load_2d_pair_hint(st + kABytes, tb, kt * 128, tok, full, pol_keep);
-          tma_load_2d_pair_hint(st + kABytes + b_sub, tb, kt * 128 + 64, tok, full, pol_keep);
-          tma_load_1d_pair(st + off_e, &tmE, (e_row + kt) * 256, full);
+          const int nk = kt + it.ks < k_end ? it.ks : k_end - kt;
+          if (leader) mbar_arrive_expect_tx(bar_full + 8 * s, nk * tx);
+          uint32_t st = sbase + s * st_bytes;
+          for (int k = kt; k < kt + nk; ++k, st += step) {
+            tma_load_2d_pair(st, &tmA, k * 64, row0, full);
+            tma_load_2d_pair_hint(st + kABytes, tb, k * 128, tok, full, pol_keep);
+            tma_load_2d_pair_hint(st + kABytes + b0, tb, k * 128 + 64, tok, full, pol_keep);
+            if (n1 > 0) {
+              tma_load_2d_pair_hint(st + kABytes + 2 * b0, &tmB1, k * 128, tok1, full, pol_keep);
+              tma_load_2d_pair_hint(st + kABytes + 2 * b0 + b1, &tmB1, k * 128 + 64, tok1, full, pol_keep);
+            }
+            tma_load_1d_pair(st + step - kEBytes, &tmE, (e_row + k) * 256, full);
+          }
           if (++s == p.stages) { s = 0; ph ^= 1; }
         }
       }
@@ -217,34 +255,43 @@ sparse_gemm_band_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_co
     // ------------------------------------------------------------ MMA issuer (even CTA of each pair)
     if (leader && elect_one()) {
       const uint16_t both = static_cast<uint16_t>(3u << even);
-      const uint32_t e_col0 = tmem_base + p.acc_bufs * p.t_full;   // metadata columns start after the accumulators
+      // metadata columns start after the accumulators
+      const uint32_t e_col0 = tmem_base + (p.tail_col > 0 ? p.tail_col + p.t_tail : p.acc_bufs * p.t_full);
       int s = 0;
       uint32_t ph = 0;
       bool ok = true;
-      uint32_t done = 0;    // items done by this pair: accumulator set = done % acc_bufs
+      uint32_t done = 0;
       for (int i = 0; i < items && ok; ++i) {
         Item it;
         if (!get_item(i, cluster_id, num_clusters, p, it)) continue;
-        const uint32_t as = p.acc_bufs == 2 ? (done & 1u) : 0u, use = p.acc_bufs == 2 ? (done >> 1) : done;
-        ++done;
-        const uint32_t idesc = make_idesc_f16(256, it.n, p.fmt, true);
-        const uint32_t d = tmem_base + as * p.t_full;
-        const uint32_t b_sub = 64u * it.n;
+        uint32_t as, use, col;
+        next_acc(p, it, done, as, use, col);
+        const int n1 = it.n - it.n0;
+        const uint32_t idesc = make_idesc_f16(256, it.n0, p.fmt, true), idesc1 = make_idesc_f16(256, n1, p.fmt, true);
+        const uint32_t d = tmem_base + col;
+        const uint32_t b0 = 64u * it.n0, b1 = 64u * n1, step = stage_bytes(it.n);
         ok = mbar_wait(bar_acce + 8 * as, (use & 1u) ^ 1u, err, p.status, 3);
         if (!ok) break;
         tc_fence_after();
-        for (int kt = k_begin; kt < k_end; ++kt) {
+        for (int kt = k_begin; kt < k_end; kt += it.ks) {
           ok = mbar_wait(bar_full + 8 * s, ph, err, p.status, 2);
           if (!ok) break;
           tc_fence_after();
-          const uint32_t st = sbase + s * st_bytes;
-          const uint32_t e_cols = e_col0 + 4 * s;
-          tc_cp_128x128b_pair(e_cols, make_smem_desc(st + off_e, 0, 128, kSwNone));
+          const int nk = kt + it.ks < k_end ? it.ks : k_end - kt;
+          uint32_t st = sbase + s * st_bytes, e_cols = e_col0 + 4 * p.ks_tail * s;
+          for (int k = kt; k < kt + nk; ++k, st += step, e_cols += 4) {
+            tc_cp_128x128b_pair(e_cols, make_smem_desc(st + step - kEBytes, 0, 128, kSwNone));
 #pragma unroll
-          for (int kb = 0; kb < 4; ++kb) {
-            const uint64_t adesc = make_smem_desc(st + kb * 32, 16, 1024, kSw128);
-            const uint64_t bdesc = make_smem_desc(st + kABytes + (kb >> 1) * b_sub + (kb & 1) * 64, 16, 1024, kSw128);
-            tc_mma_sp_f16_pair(d, adesc, bdesc, e_cols + (kb & ~1), idesc | (kb & 1), (kt > k_begin || kb > 0) ? 1u : 0u);
+            for (int kb = 0; kb < 4; ++kb) {
+              const uint64_t adesc = make_smem_desc(st + kb * 32, 16, 1024, kSw128);
+              const uint64_t bdesc = make_smem_desc(st + kABytes + (kb >> 1) * b0 + (kb & 1) * 64, 16, 1024, kSw128);
+              const uint32_t accumulate = (k > k_begin || kb > 0) ? 1u : 0u;
+              tc_mma_sp_f16_pair(d, adesc, bdesc, e_cols + (kb & ~1), idesc | (kb & 1), accumulate);
+              if (n1 > 0) {
+                const uint64_t bdesc1 = make_smem_desc(st + kABytes + 2 * b0 + (kb >> 1) * b1 + (kb & 1) * 64, 16, 1024, kSw128);
+                tc_mma_sp_f16_pair(d + it.n0, adesc, bdesc1, e_cols + (kb & ~1), idesc1 | (kb & 1), accumulate);
+              }
+            }
           }
           tc_commit_pair(bar_empty + 8 * s, both);
           if (++s == p.stages) { s = 0; ph ^= 1; }
@@ -277,12 +324,12 @@ sparse_gemm_band_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_co
     for (int i = 0; i < items && ok; ++i) {
       Item it;
       if (!get_item(i, cluster_id, num_clusters, p, it)) continue;
-      const uint32_t as = p.acc_bufs == 2 ? (done & 1u) : 0u, use = p.acc_bufs == 2 ? (done >> 1) : done;
-      ++done;
+      uint32_t as, use, col;
+      next_acc(p, it, done, as, use, col);
       ok = __all_sync(0xffffffffu, mbar_wait(bar_accf + 8 * as, use & 1u, err, p.status, 4));
       if (!ok && p.split == 1) break;
       tc_fence_after();
-      const uint32_t t_acc = tmem_base + (static_cast<uint32_t>(q * 32) << 16) + as * p.t_full;
+      const uint32_t t_acc = tmem_base + (static_cast<uint32_t>(q * 32) << 16) + col;
       const int row_w = it.m_blk * 256 + static_cast<int>(rank) * 128 + q * 32;
       const int chunks = (it.tok_end - it.tok0 + 15) / 16 < it.n / 16 ? (it.tok_end - it.tok0 + 15) / 16 : it.n / 16;
       auto load_chunk = [&](int c, uint32_t (&r)[16]) {
@@ -354,7 +401,7 @@ sparse_gemm_band_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_co
           store_chunk(r, it.tok0 + c * 16);
         }
       } else {
-        // slot of source pair s for own chunk oc, quadrant q: 2 KB of fragments, [register / 4][lane] 16 bytes each
+        // slot of each other pair for own chunk oc, quadrant q: 2 KB of fragments, [register / 4][lane] 16 bytes each
         const int own_max = (p.t_full / 16 + p.split - 1) / p.split;
         const uint32_t slot_q = static_cast<uint32_t>(q * 2048 + lane * 16);
         __syncwarp();
@@ -366,7 +413,7 @@ sparse_gemm_band_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_co
             if (owner == kpart) continue;
             load_chunk(c, r);
             const uint32_t dst = mapa_u32(sbase, 2 * owner + rank) + slot_q +
-                                 static_cast<uint32_t>((kpart * own_max + c / p.split) * 8192);
+                                 static_cast<uint32_t>(((kpart - (kpart > owner ? 1 : 0)) * own_max + c / p.split) * 8192);
 #pragma unroll
             for (int j = 0; j < 4; ++j) st_cluster_v4(dst + j * 512, &r[4 * j]);
           }
@@ -386,7 +433,7 @@ sparse_gemm_band_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_co
 #pragma unroll
                 for (int j = 0; j < 16; ++j) add_f32(r[j], own[j]);
               } else {
-                const uint32_t slot = sbase + slot_q + static_cast<uint32_t>((src * own_max + oc) * 8192);
+                const uint32_t slot = sbase + slot_q + static_cast<uint32_t>(((src - (src > kpart ? 1 : 0)) * own_max + oc) * 8192);
 #pragma unroll
                 for (int j = 0; j < 4; ++j) {
                   const uint4 v = ld_shared_v4(slot + j * 512);
@@ -472,18 +519,27 @@ int launch_band(const SparseGemmArgs& a, int split, int t, cudaStream_t stream) 
   p.n_full = q.n_full;
   p.slices = q.slices;
   p.n_tail = q.n_tail;
+  p.n0_full = t <= 256 ? t : round16(t / 2);
+  p.ks_tail = p.n_tail > 0 ? stage_bytes(t) / stage_bytes(p.t_tail) : 1;
   p.acc_bufs = (split == 1 && 2 * t + 4 * p.stages <= 512) ? 2 : 1;
-  const int used = p.acc_bufs * t + 4 * p.stages;
+  const bool tail_own = p.acc_bufs == 1 && p.n_tail > 0 && t + p.t_tail + 4 * p.stages <= 512;
+  p.tail_col = tail_own ? t : 0;
+  const int acc_cols = tail_own ? t + p.t_tail : p.acc_bufs * t;
+  while (p.ks_tail > 1 && acc_cols + 4 * p.stages * p.ks_tail > 512) --p.ks_tail;   // metadata columns of every step in flight
+  const int used = acc_cols + 4 * p.stages * p.ks_tail;
   p.tmem_cols = 32;
   while (p.tmem_cols < used) p.tmem_cols *= 2;
 
-  CUtensorMap tmA, tmB, tmBt, tmE;
+  CUtensorMap tmA, tmB, tmB1, tmBt, tmE;
   const uint64_t kc = static_cast<uint64_t>(a.K) / 2;
   if (!make_map_2d(&tmA, a.values, a.n_out, kc, kc * 2, 128, 64, CU_TENSOR_MAP_SWIZZLE_128B, a.fmt)) return kErrTensorMap;
   const uint64_t pitch = static_cast<uint64_t>(a.ldx) * 2;
-  if (!make_map_2d(&tmB, a.x, a.m_tok, a.K, pitch, t / 2, 64, CU_TENSOR_MAP_SWIZZLE_128B, a.fmt)) return kErrTensorMap;
-  tmBt = tmB;
-  if (p.t_tail != t && !make_map_2d(&tmBt, a.x, a.m_tok, a.K, pitch, p.t_tail / 2, 64, CU_TENSOR_MAP_SWIZZLE_128B, a.fmt))
+  if (!make_map_2d(&tmB, a.x, a.m_tok, a.K, pitch, p.n0_full / 2, 64, CU_TENSOR_MAP_SWIZZLE_128B, a.fmt)) return kErrTensorMap;
+  tmBt = tmB1 = tmB;
+  if (p.n0_full < t &&
+      !make_map_2d(&tmB1, a.x, a.m_tok, a.K, pitch, (t - p.n0_full) / 2, 64, CU_TENSOR_MAP_SWIZZLE_128B, a.fmt))
+    return kErrTensorMap;
+  if (p.n_tail > 0 && !make_map_2d(&tmBt, a.x, a.m_tok, a.K, pitch, p.t_tail / 2, 64, CU_TENSOR_MAP_SWIZZLE_128B, a.fmt))
     return kErrTensorMap;
   if (!make_map_1d_u64(&tmE, a.meta, meta_bytes(a.n_out, a.K) / 8, 256)) return kErrTensorMap;
 
@@ -491,38 +547,40 @@ int launch_band(const SparseGemmArgs& a, int split, int t, cudaStream_t stream) 
   const int work = p.n_full > 0 ? p.n_full : p.n_tail;
   const int clusters = (split > 1 || work < pairs) ? work : pairs;
   const size_t smem = 1024 + p.stages * stage_bytes(t) + kEpiWarps * kStagingBytes + kBarBytes;
-  return launch_dependent(sparse_gemm_band_kernel<EPI>, clusters * 2 * split, kThreads, smem, 2 * split, stream, tmA, tmB, tmBt,
-                          tmE, p);
+  return launch_dependent(sparse_gemm_band_kernel<EPI>, clusters * 2 * split, kThreads, smem, 2 * split, stream, tmA, tmB, tmB1,
+                          tmBt, tmE, p);
 }
 
 // Estimated time in us of one (split, token tile) on a GPU with num_sms SMs; constants measured on B200.
 //   K step of a t-token tile: 0.15 + 0.00102 t us (the shared-memory port, see the top of this file), wide tiles up to 12 %
 //     more where K is long (the pair kernel's factor);
 //   weights from HBM at 6.6 TB/s; the passes' K loops and that stream overlap only in part, a third of the shorter one adds;
-//   a tile with a single accumulator set (t > 240) exposes its drain between passes, 2 us;
+//   two MMAs over one weight tile (t > 256) read it from shared memory twice, 0.065 us;
+//   a tile with a single accumulator set (t > 240) exposes its drain between whole tiles, 2 us;
 //   split 2: 33 clusters of four CTAs are resident at once (of 148 SMs; clusters do not straddle the GPU's
-//   processor groups), the exchange costs 2 us + 11 ns per token column.
+//   processor groups), the exchange costs 24 ns per token column.
 double band_cost(int m_tok, int n_out, int K, int num_sms, int split, int t) {
   const int k = (K + 127) / 128, pairs = num_sms / 2 > 0 ? num_sms / 2 : 1;
   const int tiles = ((n_out + 255) / 256) * ((m_tok + t - 1) / t);
   const double dbl = k > 32 ? std::log2(k / 32.0) : 0.0, fk = 1.0 + 0.08 * (dbl < 1.5 ? dbl : 1.5);
-  auto step = [&](int n) { return (0.15 + 0.00102 * n) * (n > 160 ? fk : 1.0); };
+  auto step = [&](int n) { return (0.15 + 0.00102 * n) * (n > 160 ? fk : 1.0) + (n > 256 ? 0.065 : 0.0); };
   const double hbm = static_cast<double>(n_out) * K * 1.125 / 6.6e6;
   double comp, extra;
   if (split == 1) {
     const ItemPlan q = plan_items(tiles, t, pairs);
     const int passes = (q.n_full + pairs - 1) / pairs;
     comp = k * (passes * step(t) + (q.n_tail ? step(q.t_tail) : 0.0));
-    const bool two_sets = 2 * t + 4 * ring_stages(t) <= 512;
-    extra = 0.004 * t + (two_sets ? 0.0 : 2.0 * (passes - 1 + (q.n_tail ? 1 : 0)));
+    const int ring = 4 * ring_stages(t);
+    const bool two_sets = 2 * t + ring <= 512, tail_own = q.n_tail > 0 && t + q.t_tail + ring <= 512;
+    extra = 0.004 * t + (two_sets ? 0.0 : 2.0 * (passes - 1 + (q.n_tail > 0 && !tail_own ? 1 : 0)));
   } else {
     const int clusters = num_sms * 33 / 148 > 0 ? num_sms * 33 / 148 : 1;
     const int waves = (tiles + clusters - 1) / clusters;
     comp = waves * ((k + 1) / 2) * step(t);
-    extra = waves * (2.0 + 0.011 * t) + (waves - 1) * 3.0;
+    extra = waves * (0.024 * t - 0.6) + (waves - 1) * 5.0;
   }
   const double lo = comp < hbm ? comp : hbm, hi = comp < hbm ? hbm : comp;
-  return 4.3 + hi + lo / 3.0 + extra;
+  return 4.6 + hi + lo / 3.0 + extra;
 }
 
 }  // namespace
@@ -534,7 +592,7 @@ int pick_band_variant(int m_tok, int n_out, int K, int num_sms, double* cost_us)
   double best = 1e300;
   int pick = 0;
   const int pairs = num_sms / 2 > 0 ? num_sms / 2 : 1;
-  for (int nb = (m_tok + 255) / 256; nb <= (m_tok + 63) / 64; ++nb) {
+  for (int nb = (m_tok + kMaxTile - 1) / kMaxTile; nb <= (m_tok + 63) / 64; ++nb) {
     const int t = round16((m_tok + nb - 1) / nb);
     const int tiles = ((n_out + 255) / 256) * ((m_tok + t - 1) / t);
     for (int split = 1; split <= 2; ++split) {
@@ -552,6 +610,11 @@ int pick_band_variant(int m_tok, int n_out, int K, int num_sms, double* cost_us)
   return pick;
 }
 
+bool band_has_slices(int m_tok, int n_out, int num_sms, int variant) {
+  const int t = variant % 1000, pairs = num_sms / 2 > 0 ? num_sms / 2 : 1;
+  return variant < 7000 && t > 0 && plan_items(((n_out + 255) / 256) * ((m_tok + t - 1) / t), t, pairs).n_tail > 0;
+}
+
 int launch_sparse_gemm_band(const SparseGemmArgs& a, cudaStream_t stream) {
   const int split = a.force_bn >= 8000 ? 4 : a.force_bn >= 7000 ? 2 : 1, t = a.force_bn % 1000;
   if (a.K % 64 != 0 || a.K <= 0 || a.m_tok <= 0 || a.n_out <= 0) return kErrInvalid;
@@ -560,7 +623,7 @@ int launch_sparse_gemm_band(const SparseGemmArgs& a, cudaStream_t stream) {
        reinterpret_cast<uintptr_t>(a.y)) & 15)
     return kErrInvalid;
   if (a.out_f32 || a.peer_y != nullptr) return kErrInvalid;
-  if (t < 16 || t > 256 || t % 16 != 0 || (a.K + 127) / 128 < split) return kErrInvalid;
+  if (t < 16 || t > kMaxTile || t % 16 != 0 || (a.K + 127) / 128 < split) return kErrInvalid;
   if (a.epi == kEpiSwiGLU) {
     if (a.n_out % 32 != 0 || (a.n_out / 2) % 8 != 0) return kErrInvalid;
     return launch_band<kEpiSwiGLU>(a, split, t, stream);

@@ -14,23 +14,25 @@ def _route(M, N, K, sw=0, sms=148):
 
 
 def test_route_takes_known_forms():
-    """Band forms only from 65 to 1023 tokens, with a legal tile; from 1024 tokens a 256-row pair tile may give way to a
+    """Band forms only from 33 to 1023 tokens, with a legal tile; from 1024 tokens a 256-row pair tile may give way to a
     512-row one; up to 8 tokens on few row tiles the slab kernel and split K may swap; everything else is the plan."""
     plan = _lib.lib().sfb200_debug_plan_gemm
     for sms in (148, 132, 64, 2):
         for N, K in ((4096, 4096), (22016, 4096), (4096, 11008), (57344, 8192), (8, 64), (392, 1088), (1024, 512)):
-            for M in (1, 2, 5, 8, 32, 64, 65, 100, 160, 161, 256, 257, 300, 512, 777, 1023, 1024, 5000):
+            for M in (1, 2, 5, 8, 32, 33, 64, 65, 100, 160, 161, 256, 257, 300, 512, 777, 1023, 1024, 5000):
                 v = _route(M, N, K, 0, sms)
                 if v >= 6000:
                     t = v % 1000
-                    assert 64 < M < 1024 and v < 8000 and 16 <= t <= 256 and t % 16 == 0, (M, N, K, sms, v)
+                    assert 32 < M < 1024 and v < 8000 and 16 <= t <= 400 and t % 16 == 0, (M, N, K, sms, v)
                     assert v < 7000 or K >= 1024 - 127, (M, N, K, sms, v)
                 elif M <= 8 and v != plan(M, N, K, 0, sms):
                     assert v in (8, 3032, 4032) and plan(M, N, K, 0, sms) in (8, 3032, 4032), (M, N, K, sms, v)
                 elif M >= 1024 and 1192 <= plan(M, N, K, 0, sms) <= 1240:
                     assert v in (1192, 1208, 1224, 1240, 5192, 5208, 5224, 5240), (M, N, K, sms, v)
+                elif 32 < M <= 128:
+                    assert v in (plan(M, N, K, 0, sms), 64), (M, N, K, sms, v)
                 else:
-                    assert v == plan(M, N, K, 0, sms) and not 64 < M <= 160, (M, N, K, sms, v)
+                    assert v == plan(M, N, K, 0, sms) and not 128 < M <= 160, (M, N, K, sms, v)
     assert _route(4096, 22016, 4096, 1) == 5240 and _route(1500, 4096, 4096) == 5192
     assert _route(150, 4096, 11008) == 7080 and _route(150, 22016, 4096, 1) == 6160 and _route(0, 8, 64) == 0
 
@@ -48,9 +50,11 @@ def _close(y, ref):
 
 # (M, N, K, variant): one tile; rows below a tile; K with a 64-wide tail; uneven K slices; a ragged last token block;
 # several passes with both accumulator sets; left-over tiles cut into slices (172 = 148 + 24 tiles, 3 slices; 86 = 74 + 12,
-# 6 slices, the last one empty of tokens); one wide tile with a single accumulator set
+# 6 slices, the last one empty of tokens); tiles above 256 tokens (two MMAs of unequal width, slices in columns of their own,
+# several K steps of a slice per ring stage with a remainder, the largest exchange); one accumulator set over several passes
 CASES = [(64, 256, 256, 6064), (16, 8, 64, 6016), (300, 392, 1088, 6160), (300, 392, 1088, 7160), (300, 392, 1088, 8160),
-         (33, 1160, 2048, 8048), (500, 520, 2048, 7256), (2000, 6136, 256, 6240), (300, 22016, 256, 6160),
+         (300, 22016, 256, 6304), (777, 11008, 384, 6400), (270, 256, 1088, 7272), (777, 520, 2048, 7400), (600, 392, 1088, 8304),
+         (350, 264, 192, 6352), (1200, 20000, 128, 6400), (33, 1160, 2048, 8048), (500, 520, 2048, 7256), (2000, 6136, 256, 6240), (300, 22016, 256, 6160),
          (150, 22016, 256, 6160), (1, 264, 1024, 7016), (700, 20000, 128, 6256)]
 
 
