@@ -126,10 +126,10 @@ int launch_sparse_gemm_splitk(const SparseGemmArgs& a, int split, cudaStream_t s
 int splitk_factor(int m_tok, int n_out, int K, int num_sms);
 int splitk_token_tile(int m_tok);
 
-// CTA-pair kernel for token counts between decode and prefill: token tile t (a multiple of 16 up to 256), K split over
-// `split` pairs of a cluster.  force_bn = 6000 + t (split 1), 7000 + t (split 2) or 8000 + t (split 4).
+// CTA-pair kernel for token counts between decode and prefill: token tile t (a multiple of 16 up to 400), K split over
+// `split` pairs of a cluster.  force_bn = 6000 + t (split 1), 7000 + t (split 2), 9000 + t (split 3) or 8000 + t (split 4).
 int launch_sparse_gemm_band(const SparseGemmArgs& a, cudaStream_t stream);
-// The form of that kernel estimated fastest for a shape (6000 + t or 7000 + t) and its estimated time in us.
+// The form of that kernel estimated fastest for a shape and its estimated time in us.
 int pick_band_variant(int m_tok, int n_out, int K, int num_sms, double* cost_us = nullptr);
 // Whether a split-1 form cuts left-over tiles into token slices for a shape.
 bool band_has_slices(int m_tok, int n_out, int num_sms, int variant);

@@ -442,12 +442,12 @@ int plan_sparse_gemm(int m_tok, int n_out, int K, int epi, int num_sms) {
 }
 
 // Estimated time in us of the single-CTA 64-token tiles: a 128-wide K step costs 0.215 us, the weights stream at 6.6 TB/s and
-// a third of the shorter of the two adds (11008 x 4096 at 64 tokens 13.5 us, 6000 x 3072 at 72 tokens 8.7 us, 8192 x 8192 at 128
+// 0.45 of the shorter of the two adds (11008 x 4096 at 64 tokens 13.5 us, 6000 x 3072 at 72 tokens 8.7 us, 8192 x 8192 at 128
 // tokens 22.0 us measured).
 double tile64_cost(int m_tok, int n_out, int K, int num_sms) {
   const int tiles = ((n_out + 127) / 128) * ((m_tok + 63) / 64);
   const double comp = ((tiles + num_sms - 1) / num_sms) * ((K + 127) / 128) * 0.215, hbm = n_out * (K * 1.125) / 6.6e6;
-  return 3.6 + (comp > hbm ? comp + hbm / 3.0 : hbm + comp / 3.0);
+  return 2.6 + (comp > hbm ? comp + 0.45 * hbm : hbm + 0.45 * comp);
 }
 
 // From 33 to 1023 tokens the band kernel (sparse_gemm_sm100_band.cu) is weighed against the fixed tiles by estimated time.

@@ -14,7 +14,7 @@
 //     than pairs) are cut into token slices, as many as the idle pairs allow, so the last pass is short.  A slice packs as
 //     many K steps into a ring stage as a whole tile's stage has room for: with one, the three stages of a 304-token
 //     ring kept 78 KB of a slice in flight and its step took 0.4 us of latency (22016 x 4096 at 300 tokens 40.3 us, now 36.9);
-//   * split 2 or 4 (few row tiles): a cluster of 2 or 4 pairs shares one tile, each pair streaming a slice of K.  The fp32
+//   * split 2, 3 or 4 (few row tiles): a cluster of that many pairs shares one tile, each pair streaming a slice of K.  The fp32
 //     accumulators are summed through distributed shared memory: pair p owns the 16-token chunks c with c % split == p,
 //     the others store theirs into its shared memory (the drained operand ring) as register fragments, 512 contiguous
 //     bytes per store instruction, and the owner adds them in pair order.  No scratch in global memory, no
@@ -23,7 +23,7 @@
 // Measured (B200, steady load at the power limit, fixed tiles before -> now): 4096 x 11008 at 150 / 300 / 400 tokens 34.2 / 34.2 /
 // 36.2 -> 18.5 / 24.3 / 28.0 us; 22016 x 4096 (SiLU.mul) at 72 / 150 / 300 / 400 tokens 27.9 / 33.1 / 47.8 / 49.1 -> 25.5 / 28.3 /
 // 36.9 / 44.5 us; 8192 x 8192 at 520 tokens 55.5 -> 42.0 us; 57344 x 8192 at 300 tokens 219.7 -> 176.8 us.  Evict-last token loads and
-// evict-first stores are 3-10 % of that.  Split 4 and slices first measured slower (below).
+// evict-first stores are 3-10 % of that.  Split 3 against split 2: 4096 x 11008 at 96 / 150 tokens 18.3 / 19.2 -> 16.0 / 17.6 us.
 //
 // Warps: warp 0 = TMA producer, warp 1 = MMA issuer / tensor-memory owner, warps 2 ... 17 = epilogue.
 // All loads are plain per-CTA TMA copies.
@@ -69,7 +69,8 @@ struct BandParams {
   int split;              // pairs per cluster = K slices
   int t_full, t_tail;     // tokens of a full item / of a slice of a left-over tile
   int n0_full;            // columns of a full item's first MMA (the rest, if any, is a second one over the same weights)
-  int ks_tail;            // K steps per ring stage of a slice: what fits the stage of a full item
+  int ks_tail;            // K steps per ring stage of a slice
+  int stage_stride;       // bytes of a ring stage: one K step of a whole tile, ks_tail of a slice
   int tail_col;           // > 0: slices accumulate in columns of their own, from this one on
   int num_n_blks;         // token blocks of t_full
   int n_full;             // items [0, n_full) are whole tiles, the rest slices of the tiles from n_full on
@@ -149,7 +150,7 @@ sparse_gemm_band_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_co
   // the same offset in every CTA of the cluster: the dynamic shared memory base is identical
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
   const uint32_t sbase = smem_u32(smem);
-  const uint32_t st_bytes = static_cast<uint32_t>(stage_bytes(p.t_full));
+  const uint32_t st_bytes = static_cast<uint32_t>(p.stage_stride);
   const uint32_t staging = sbase + p.stages * st_bytes;
   const uint32_t bar_full = staging + kEpiWarps * kStagingBytes;   // used in the even CTA of the pair only
   const uint32_t bar_empty = bar_full + 8 * kMaxStages;            // both CTAs
@@ -469,6 +470,28 @@ sparse_gemm_band_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_co
 
 int round16(int v) { return (v + 15) & ~15; }
 
+// Ring geometry.  A slice packs ks K steps into a stage; the stage is made larger than a whole tile's K step where that
+// puts more bytes of a slice in flight without taking the ring below four stages (three for tiles above 256 tokens).  At one
+// step per stage the slices of a 160-token ring (5 x 22 KB in flight) ran at 0.30 us a step, bound by latency.
+struct Ring {
+  int stages, ks, stride;
+};
+Ring plan_ring(int t, int t_tail, bool slices) {
+  Ring best{ring_stages(t), 1, stage_bytes(t)};
+  if (!slices) return best;
+  int most = best.stages * stage_bytes(t_tail);
+  for (int ks = 2; ks <= 4; ++ks) {
+    const int need = ks * stage_bytes(t_tail), stride = need > stage_bytes(t) ? need : stage_bytes(t);
+    int stages = kRingBytes / stride < kMaxStages ? kRingBytes / stride : kMaxStages;
+    if (stages < (t > 256 ? 3 : 4)) break;
+    if (stages * need > most) {
+      most = stages * need;
+      best = Ring{stages, ks, stride};
+    }
+  }
+  return best;
+}
+
 // Work items of a split-1 launch: tiles that fill whole passes over the pairs, then the left-over tiles cut into
 // token slices so that one more, shorter pass covers them.
 struct ItemPlan {
@@ -509,7 +532,6 @@ int launch_band(const SparseGemmArgs& a, int split, int t, cudaStream_t stream) 
   p.split = split;
   p.t_full = t;
   p.num_n_blks = (a.m_tok + t - 1) / t;
-  p.stages = ring_stages(t);
   p.fmt = a.fmt;
   p.act = a.act;
   const int tiles = ((a.n_out + 255) / 256) * p.num_n_blks;
@@ -520,7 +542,10 @@ int launch_band(const SparseGemmArgs& a, int split, int t, cudaStream_t stream) 
   p.slices = q.slices;
   p.n_tail = q.n_tail;
   p.n0_full = t <= 256 ? t : round16(t / 2);
-  p.ks_tail = p.n_tail > 0 ? stage_bytes(t) / stage_bytes(p.t_tail) : 1;
+  const Ring ring = plan_ring(t, p.t_tail, p.n_tail > 0);
+  p.stages = ring.stages;
+  p.ks_tail = ring.ks;
+  p.stage_stride = ring.stride;
   p.acc_bufs = (split == 1 && 2 * t + 4 * p.stages <= 512) ? 2 : 1;
   const bool tail_own = p.acc_bufs == 1 && p.n_tail > 0 && t + p.t_tail + 4 * p.stages <= 512;
   p.tail_col = tail_own ? t : 0;
@@ -546,9 +571,17 @@ int launch_band(const SparseGemmArgs& a, int split, int t, cudaStream_t stream) 
   // split > 1: one cluster per tile; split 1: persistent pairs (a plan with slices fills whole passes before them)
   const int work = p.n_full > 0 ? p.n_full : p.n_tail;
   const int clusters = (split > 1 || work < pairs) ? work : pairs;
-  const size_t smem = 1024 + p.stages * stage_bytes(t) + kEpiWarps * kStagingBytes + kBarBytes;
+  const size_t smem = 1024 + static_cast<size_t>(p.stages) * p.stage_stride + kEpiWarps * kStagingBytes + kBarBytes;
   return launch_dependent(sparse_gemm_band_kernel<EPI>, clusters * 2 * split, kThreads, smem, 2 * split, stream, tmA, tmB, tmB1,
                           tmBt, tmE, p);
+}
+
+// Clusters of 2 * split CTAs that are resident at once: a cluster does not straddle the GPU's processor groups, and on the 148
+// SMs of a B200 74, 33, 22 and 15 fit (cudaOccupancyMaxActiveClusters).
+int clusters_resident(int split, int num_sms) {
+  const int of148[5] = {0, 74, 33, 22, 15};
+  const int n = num_sms * of148[split] / 148;
+  return n > 0 ? n : 1;
 }
 
 // Estimated time in us of one (split, token tile) on a GPU with num_sms SMs; constants measured on B200.
@@ -557,27 +590,28 @@ int launch_band(const SparseGemmArgs& a, int split, int t, cudaStream_t stream) 
 //   weights from HBM at 6.6 TB/s; the passes' K loops and that stream overlap only in part, a third of the shorter one adds;
 //   two MMAs over one weight tile (t > 256) read it from shared memory twice, 0.065 us;
 //   a tile with a single accumulator set (t > 240) exposes its drain between whole tiles, 2 us;
-//   split 2: 33 clusters of four CTAs are resident at once (of 148 SMs; clusters do not straddle the GPU's
-//   processor groups), the exchange costs 24 ns per token column.
+//   split K: the exchange costs 0.4 us + 10 ns per token column; with more than three quarters of the pairs at work on the few row tiles
+//     of such a shape a step takes 15 % longer (one partly filled pass of split 1: 7 %).
 double band_cost(int m_tok, int n_out, int K, int num_sms, int split, int t) {
   const int k = (K + 127) / 128, pairs = num_sms / 2 > 0 ? num_sms / 2 : 1;
   const int tiles = ((n_out + 255) / 256) * ((m_tok + t - 1) / t);
-  const double dbl = k > 32 ? std::log2(k / 32.0) : 0.0, fk = 1.0 + 0.08 * (dbl < 1.5 ? dbl : 1.5);
+  const double ks = (k + split - 1) / split, dbl = ks > 32 ? std::log2(ks / 32.0) : 0.0, fk = 1.0 + 0.08 * (dbl < 1.5 ? dbl : 1.5);
   auto step = [&](int n) { return (0.15 + 0.00102 * n) * (n > 160 ? fk : 1.0) + (n > 256 ? 0.065 : 0.0); };
   const double hbm = static_cast<double>(n_out) * K * 1.125 / 6.6e6;
   double comp, extra;
   if (split == 1) {
     const ItemPlan q = plan_items(tiles, t, pairs);
     const int passes = (q.n_full + pairs - 1) / pairs;
-    comp = k * (passes * step(t) + (q.n_tail ? step(q.t_tail) : 0.0));
+    const double crowd = (tiles <= pairs && 4 * tiles > 3 * pairs) ? 1.07 : 1.0;
+    comp = k * (passes * step(t) + (q.n_tail ? step(q.t_tail) : 0.0)) * crowd;
     const int ring = 4 * ring_stages(t);
     const bool two_sets = 2 * t + ring <= 512, tail_own = q.n_tail > 0 && t + q.t_tail + ring <= 512;
     extra = 0.004 * t + (two_sets ? 0.0 : 2.0 * (passes - 1 + (q.n_tail > 0 && !tail_own ? 1 : 0)));
   } else {
-    const int clusters = num_sms * 33 / 148 > 0 ? num_sms * 33 / 148 : 1;
-    const int waves = (tiles + clusters - 1) / clusters;
-    comp = waves * ((k + 1) / 2) * step(t);
-    extra = waves * (0.024 * t - 0.6) + (waves - 1) * 5.0;
+    const int resident = clusters_resident(split, num_sms), waves = (tiles + resident - 1) / resident;
+    const double crowd = 4 * tiles * split > 3 * pairs ? 1.15 : 1.0;
+    comp = waves * ks * step(t) * crowd;
+    extra = 0.4 + 0.010 * t + (waves - 1) * 5.0;
   }
   const double lo = comp < hbm ? comp : hbm, hi = comp < hbm ? hbm : comp;
   return 4.6 + hi + lo / 3.0 + extra;
@@ -585,24 +619,23 @@ double band_cost(int m_tok, int n_out, int K, int num_sms, int split, int t) {
 
 }  // namespace
 
-// Cheapest form for a shape: split 1 or 2 and the token tile that cuts the tokens into equal blocks.  (Split 4 is not a
-// candidate: only 15 clusters of eight CTAs fit the GPU at once, one fewer than the 16 row tiles of a 4096-row weight, and
-// it measured 1.3-2 x slower than split 2 there.)
+// Cheapest form for a shape: split 1 ... 4 and the token tile that cuts the tokens into equal blocks.
 int pick_band_variant(int m_tok, int n_out, int K, int num_sms, double* cost_us) {
+  constexpr int kForm[5] = {0, 6000, 7000, 9000, 8000};
   double best = 1e300;
   int pick = 0;
   const int pairs = num_sms / 2 > 0 ? num_sms / 2 : 1;
   for (int nb = (m_tok + kMaxTile - 1) / kMaxTile; nb <= (m_tok + 63) / 64; ++nb) {
     const int t = round16((m_tok + nb - 1) / nb);
     const int tiles = ((n_out + 255) / 256) * ((m_tok + t - 1) / t);
-    for (int split = 1; split <= 2; ++split) {
-      if (split == 2 && (K + 127) / 128 < 8) continue;
+    for (int split = 1; split <= 4; ++split) {
+      if (split > 1 && (K + 127) / 128 < 4 * split) continue;      // at least K = 512 per slice
       // fewer tiles than half the pairs: more, narrower token blocks do what slicing every tile would, with a deeper ring
       if (split == 1 && 2 * tiles <= pairs && t > 64) continue;
       const double c = band_cost(m_tok, n_out, K, num_sms, split, t);
       if (c < best) {
         best = c;
-        pick = 5000 + 1000 * split + t;
+        pick = kForm[split] + t;
       }
     }
   }
@@ -616,7 +649,7 @@ bool band_has_slices(int m_tok, int n_out, int num_sms, int variant) {
 }
 
 int launch_sparse_gemm_band(const SparseGemmArgs& a, cudaStream_t stream) {
-  const int split = a.force_bn >= 8000 ? 4 : a.force_bn >= 7000 ? 2 : 1, t = a.force_bn % 1000;
+  const int split = a.force_bn >= 9000 ? 3 : a.force_bn >= 8000 ? 4 : a.force_bn >= 7000 ? 2 : 1, t = a.force_bn % 1000;
   if (a.K % 64 != 0 || a.K <= 0 || a.m_tok <= 0 || a.n_out <= 0) return kErrInvalid;
   if (a.n_out % 8 != 0 || a.ldx % 8 != 0 || a.ldy % 8 != 0) return kErrInvalid;
   if ((reinterpret_cast<uintptr_t>(a.x) | reinterpret_cast<uintptr_t>(a.values) | reinterpret_cast<uintptr_t>(a.meta) |

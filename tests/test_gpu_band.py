@@ -1,4 +1,4 @@
-"""CTA-pair GEMM for token counts between decode and prefill (force 6000 / 7000 / 8000 + token tile = K split over 1 / 2 / 4
+"""CTA-pair GEMM for token counts between decode and prefill (force 6000 / 7000 / 9000 / 8000 + token tile = K split over 1 / 2 / 3 / 4
 pairs), against an fp32 matmul on the decompressed weight and against a fixed-tile kernel on the same call."""
 import pytest
 import torch
@@ -23,8 +23,8 @@ def test_route_takes_known_forms():
                 v = _route(M, N, K, 0, sms)
                 if v >= 6000:
                     t = v % 1000
-                    assert 32 < M < 1024 and v < 8000 and 16 <= t <= 400 and t % 16 == 0, (M, N, K, sms, v)
-                    assert v < 7000 or K >= 1024 - 127, (M, N, K, sms, v)
+                    assert 32 < M < 1024 and v < 10000 and 16 <= t <= 400 and t % 16 == 0, (M, N, K, sms, v)
+                    assert v < 7000 or K > 512 * {7: 2, 9: 3, 8: 4}[v // 1000] - 128, (M, N, K, sms, v)
                 elif M <= 8 and v != plan(M, N, K, 0, sms):
                     assert v in (8, 3032, 4032) and plan(M, N, K, 0, sms) in (8, 3032, 4032), (M, N, K, sms, v)
                 elif M >= 1024 and 1192 <= plan(M, N, K, 0, sms) <= 1240:
@@ -34,7 +34,7 @@ def test_route_takes_known_forms():
                 else:
                     assert v == plan(M, N, K, 0, sms) and not 128 < M <= 160, (M, N, K, sms, v)
     assert _route(4096, 22016, 4096, 1) == 5240 and _route(1500, 4096, 4096) == 5192
-    assert _route(150, 4096, 11008) == 7080 and _route(150, 22016, 4096, 1) == 6160 and _route(0, 8, 64) == 0
+    assert _route(150, 4096, 11008) == 9160 and _route(150, 22016, 4096, 1) == 6160 and _route(0, 8, 64) == 0
 
 
 @pytest.fixture
@@ -53,6 +53,7 @@ def _close(y, ref):
 # 6 slices, the last one empty of tokens); tiles above 256 tokens (two MMAs of unequal width, slices in columns of their own,
 # several K steps of a slice per ring stage with a remainder, the largest exchange); one accumulator set over several passes
 CASES = [(64, 256, 256, 6064), (16, 8, 64, 6016), (300, 392, 1088, 6160), (300, 392, 1088, 7160), (300, 392, 1088, 8160),
+         (300, 392, 1088, 9160), (77, 1160, 2048, 9080), (777, 520, 2048, 9400), (400, 22016, 640, 6208), (512, 28672, 256, 6256),
          (300, 22016, 256, 6304), (777, 11008, 384, 6400), (270, 256, 1088, 7272), (777, 520, 2048, 7400), (600, 392, 1088, 8304),
          (350, 264, 192, 6352), (1200, 20000, 128, 6400), (33, 1160, 2048, 8048), (500, 520, 2048, 7256), (2000, 6136, 256, 6240), (300, 22016, 256, 6160),
          (150, 22016, 256, 6160), (1, 264, 1024, 7016), (700, 20000, 128, 6256)]
@@ -99,7 +100,7 @@ def test_band_kernel_swiglu(force, M, I, K, v, dt):
 
 
 @pytest.mark.gpu
-@pytest.mark.parametrize("v", [6128, 7128, 8128])
+@pytest.mark.parametrize("v", [6128, 7128, 8128, 9128, 9336])
 def test_band_kernel_identity_is_exact(force, v):
     """One-hot activations return the pruned weight bit for bit, whichever pair owns a chunk."""
     w = (torch.randn(4096, 1024, device="cuda") * 0.02).to(torch.bfloat16)
