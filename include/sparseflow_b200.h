@@ -87,12 +87,6 @@ SFB200_API int sfb200_prune_compress_24(const void* dense, int rows, int K, int 
                                         int tie, void* values, void* meta, void* ref_codes,
                                         void* pruned, void* stream);
 
-/* Compression of a weight that should be 2:4 already into the container of sfb200_blob_* (blob: device, 16-byte aligned,
- * sfb200_blob_bytes(rows, K) bytes): header, values, padding and metadata in one pass.  *not_24_dev (device) becomes 1 if a
- * group of four has more than two non-zeros, else 0.  K a multiple of 16, dense 16-byte aligned, ld a multiple of 8. */
-SFB200_API int sfb200_compress_blob_checked(const void* dense, int rows, int K, int ld, int dtype, int tie, void* blob,
-                                            int* not_24_dev, void* stream);
-
 /*
  * Same, for the fused gate|up weight of the gated FFN: reads gate[I, K] and up[I, K] and emits
  * the 2*I-row matrix whose rows alternate in blocks of 16 (16 gate rows, the matching 16 up
@@ -103,6 +97,12 @@ SFB200_API int sfb200_compress_blob_checked(const void* dense, int rows, int K, 
 SFB200_API int sfb200_prune_compress_gate_up(const void* gate, const void* up, int I, int K, int ld,
                                              int dtype, int tie, void* values, void* meta,
                                              void* stream);
+
+/* Compression of a weight that should be 2:4 already into the container of sfb200_blob_* (blob: device, 16-byte aligned,
+ * sfb200_blob_bytes(rows, K) bytes): header, values, padding and metadata in one pass.  *not_24_dev (device) becomes 1 if a
+ * group of four has more than two non-zeros, else 0.  K a multiple of 16, dense 16-byte aligned, ld a multiple of 8. */
+SFB200_API int sfb200_compress_blob_checked(const void* dense, int rows, int K, int ld, int dtype, int tie, void* blob,
+                                            int* not_24_dev, void* stream);
 
 /* is_valid_dev (device int) := 1 iff every group of four has <= 2 non-zeros.
  * Device-pointer form of sparseflow_validate_2_4 (include/sparseflow/c_api.h:171-176). */
@@ -140,6 +140,12 @@ SFB200_API int sfb200_sparse_gemm_f32out(const void* x, int ldx, const void* val
 SFB200_API int sfb200_sparse_gemm_swiglu(const void* x, int ldx, const void* values_gu,
                                          const void* meta_gu, void* h, int ldh, int M, int I, int K,
                                          int dtype, void* stream);
+
+/* The same with a bias on the gate and / or the up features ([I] each, dtype as the activations; null = none), added to the
+ * fp32 sums before SiLU.mul. */
+SFB200_API int sfb200_sparse_gemm_swiglu_bias(const void* x, int ldx, const void* values_gu, const void* meta_gu,
+                                              const void* gate_bias, const void* up_bias, void* h, int ldh, int M, int I,
+                                              int K, int dtype, void* stream);
 
 /* out[r, c] = silu(gate[r, c]) * up[r, c], fp32 math (sparseflow/kernels/fused_silu_mul.py:33-57).
  * Unfused variant, kept for the dense branch of the shape gate. */

@@ -70,6 +70,7 @@ def lib() -> C.CDLL:
     L.sfb200_decompress_24.argtypes = [vp, vp, i, i, vp, i, vp]
     L.sfb200_sparse_gemm.argtypes = [vp, i, vp, vp, vp, i, i, i, i, i, vp, i, vp]
     L.sfb200_sparse_gemm_swiglu.argtypes = [vp, i, vp, vp, vp, i, i, i, i, i, vp]
+    L.sfb200_sparse_gemm_swiglu_bias.argtypes = [vp, i, vp, vp, vp, vp, vp, i, i, i, i, i, vp]
     L.sfb200_silu_mul.argtypes = [vp, i, vp, i, vp, i, i, i, i, vp]
     L.sfb200_ffn_forward.argtypes = [C.POINTER(FFNWeights), vp, i, vp, vp, i, i, vp]
     L.sfb200_ffn_forward_host.argtypes = [C.POINTER(FFNWeights), vp, vp, i, vp]

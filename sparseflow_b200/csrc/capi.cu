@@ -212,7 +212,7 @@ int sfb200_decompress_24(const void* values, const void* meta, int rows, int K, 
 
 static int run_gemm(DeviceState* s, const void* x, int ldx, const void* values, const void* meta,
                     void* y, int ldy, int M, int N, int K, int dtype, const void* bias, int act,
-                    int epi, int force_bn, cudaStream_t st) {
+                    int epi, int force_bn, cudaStream_t st, const void* bias_up = nullptr) {
   if (!x || !values || !meta || !y) return kErrInvalid;
   if (dtype != kF16 && dtype != kBF16) return kErrInvalid;
   SparseGemmArgs a{};
@@ -221,6 +221,7 @@ static int run_gemm(DeviceState* s, const void* x, int ldx, const void* values, 
   a.meta = meta;
   a.y = y;
   a.bias = bias;
+  a.bias_up = bias_up;
   a.status = s->status;
   a.m_tok = M;
   a.n_out = N;
@@ -254,6 +255,16 @@ int sfb200_sparse_gemm_swiglu(const void* x, int ldx, const void* values_gu, con
   Range r("sfb200.gate_up_gemm");
   return run_gemm(s, x, ldx, values_gu, meta_gu, h, ldh, M, 2 * I, K, dtype, nullptr, kActNone,
                   kEpiSwiGLU, 0, static_cast<cudaStream_t>(stream));
+}
+
+int sfb200_sparse_gemm_swiglu_bias(const void* x, int ldx, const void* values_gu, const void* meta_gu, const void* gate_bias,
+                                   const void* up_bias, void* h, int ldh, int M, int I, int K, int dtype, void* stream) {
+  int err = kOk;
+  DeviceState* s = device_state(&err);
+  if (!s) return err;
+  Range r("sfb200.gate_up_gemm");
+  return run_gemm(s, x, ldx, values_gu, meta_gu, h, ldh, M, 2 * I, K, dtype, gate_bias, kActNone, kEpiSwiGLU, 0,
+                  static_cast<cudaStream_t>(stream), up_bias);
 }
 
 int sfb200_silu_mul(const void* gate, int ld_gate, const void* up, int ld_up, void* out, int ld_out,

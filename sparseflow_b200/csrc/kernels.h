@@ -59,7 +59,8 @@ struct SparseGemmArgs {
   const void* values;     // [n_out, K/2]
   const void* meta;       // tiled metadata of the n_out x K weight
   void* y;                // kEpiStore: [m_tok, n_out];  kEpiSwiGLU: [m_tok, n_out/2]; pitch ldy
-  const void* bias;       // [n_out] or null (kEpiStore only)
+  const void* bias;       // kEpiStore: [n_out] or null.  kEpiSwiGLU: bias of the gate rows, [n_out / 2] or null
+  const void* bias_up;    // kEpiSwiGLU: bias of the up rows, [n_out / 2] or null
   int* status;            // device status word
   int m_tok, n_out, K;
   int ldx, ldy;

@@ -148,4 +148,23 @@ __device__ __forceinline__ float silu_mul(uint32_t g, uint32_t u) {
   return (gf * __fdividef(1.f, 1.f + __expf(-gf))) * __uint_as_float(u);
 }
 
+__device__ __forceinline__ float silu_mul_bias(uint32_t g, uint32_t u, float bias_g, float bias_u) {
+  const float gf = __uint_as_float(g) + bias_g;
+  return (gf * __fdividef(1.f, 1.f + __expf(-gf))) * (__uint_as_float(u) + bias_u);
+}
+// SiLU.mul epilogue: bias of gate features f = row_w / 2 + g, f + 8 (b0, b1) and of the matching up features (b2, b3), for a
+// warp whose 32 interleaved rows start at row_w.  Either bias may be null.
+__device__ __forceinline__ void load_gate_up_bias(const void* gate, const void* up, int row_w, int g, int n_out, int fmt, float& b0,
+                                                  float& b1, float& b2, float& b3) {
+  const int f = row_w / 2 + g;
+  if (row_w >= n_out) return;      // whole blocks of 32 rows
+  if (gate != nullptr) {
+    b0 = bias_at(gate, f, fmt);
+    b1 = bias_at(gate, f + 8, fmt);
+  }
+  if (up != nullptr) {
+    b2 = bias_at(up, f, fmt);
+    b3 = bias_at(up, f + 8, fmt);
+  }
+}
 }  // namespace sfb200

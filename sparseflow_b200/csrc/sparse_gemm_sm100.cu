@@ -31,7 +31,8 @@ namespace {
 
 struct GemmParams {
   const uint32_t* meta;   // [row_tiles][k_tiles][128][4]
-  const void* bias;       // per out feature, 16-bit type, or null
+  const void* bias;       // as SparseGemmArgs
+  const void* bias_up;
   int* status;            // device status word
   int n_out;              // weight rows
   int m_tok;              // tokens
@@ -254,6 +255,11 @@ sparse_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
         const int o = m_blk * C::BM + q * 32 + lane;
         if (o < p.n_out) bias_v = from_bits16(static_cast<const uint16_t*>(p.bias)[o], p.fmt);
       }
+      if (C::EPI == kEpiSwiGLU) {      // lanes 0..15 hold gate features, 16..31 the matching up features
+        const uint16_t* src = static_cast<const uint16_t*>(lane < 16 ? p.bias : p.bias_up);
+        const int row = m_blk * C::BM + q * 32;
+        if (src != nullptr && row < p.n_out) bias_v = from_bits16(src[row / 2 + (lane & 15)], p.fmt);
+      }
       for (int c = 0; c < n_chunks; ++c) {
         tmem_ld_32x32(t_acc + c * 32, r);
         tmem_ld_wait();
@@ -282,6 +288,10 @@ sparse_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
           // j, the upper half-warp token j+1.
           const bool upper = lane >= 16;
           uint16_t* scol = reinterpret_cast<uint16_t*>(stage) + q * 16 + (lane & 15);
+          if (p.bias != nullptr || p.bias_up != nullptr) {
+#pragma unroll
+            for (int j = 0; j < 32; ++j) r[j] = __float_as_uint(__uint_as_float(r[j]) + bias_v);
+          }
 #pragma unroll
           for (int j = 0; j < 32; j += 2) {
             const uint32_t send = upper ? r[j] : r[j + 1];
@@ -347,6 +357,7 @@ int launch_cfg(const SparseGemmArgs& a, cudaStream_t stream) {
   GemmParams p;
   p.meta = static_cast<const uint32_t*>(a.meta);
   p.bias = a.bias;
+  p.bias_up = a.bias_up;
   p.status = a.status;
   p.n_out = a.n_out;
   p.m_tok = a.m_tok;

@@ -38,7 +38,8 @@ namespace sfb200 {
 namespace {
 
 struct PairParams {
-  const void* bias;
+  const void* bias;       // as SparseGemmArgs
+  const void* bias_up;
   void* y;
   int* status;
   int n_out, m_tok, K, ldy;
@@ -405,7 +406,11 @@ __device__ __forceinline__ void pair_kernel_body(const CUtensorMap& tmA, const C
           // half 0 = 16 gate rows, half 1 = the 16 matching up rows: pairing is in-thread
           // (the output type is tested once per chunk, not once per value: the drain is a chain of dependent
           // instructions and every branch inside it costs latency that nothing hides)
-          if (p.fmt == 1)
+          if (p.bias != nullptr || p.bias_up != nullptr) {
+            auto f = [&](int i, float bg, float bu) { return silu_mul_bias(a[i], b[i], bg, bu); };
+            stmatrix_x4_trans(stage + st_off, pack16(f(0, b0, b2), f(1, b0, b2), p.fmt), pack16(f(2, b1, b3), f(3, b1, b3), p.fmt),
+                              pack16(f(4, b0, b2), f(5, b0, b2), p.fmt), pack16(f(6, b1, b3), f(7, b1, b3), p.fmt));
+          } else if (p.fmt == 1)
             stmatrix_x4_trans(stage + st_off, pack16(silu_mul(a[0], b[0]), silu_mul(a[1], b[1]), 1),
                               pack16(silu_mul(a[2], b[2]), silu_mul(a[3], b[3]), 1),
                               pack16(silu_mul(a[4], b[4]), silu_mul(a[5], b[5]), 1),
@@ -498,6 +503,7 @@ __device__ __forceinline__ void pair_kernel_body(const CUtensorMap& tmA, const C
           if (row_w + g + 16 < p.n_out) b2 = bias_at(p.bias, row_w + g + 16, p.fmt);
           if (row_w + g + 24 < p.n_out) b3 = bias_at(p.bias, row_w + g + 24, p.fmt);
         }
+        if (C::EPI == kEpiSwiGLU) load_gate_up_bias(p.bias, p.bias_up, row_w, g, p.n_out, p.fmt, b0, b1, b2, b3);
         // two register sets in turn: the loads of chunk c + 1 are in flight while chunk c is converted and stored
         uint32_t ra[8], rb[8], sa[8], sb[8];
         auto load_chunk = [&](int c, uint32_t (&lo)[8], uint32_t (&hi)[8]) {
@@ -566,6 +572,7 @@ int launch_pair_cfg(const SparseGemmArgs& a, cudaStream_t stream) {
   if (!make_map_1d_u64(&tmE, a.meta, meta_bytes(a.n_out, a.K) / 8, 256)) return kErrTensorMap;
   PairParams p;
   p.bias = a.bias;
+  p.bias_up = a.bias_up;
   p.y = a.y;
   p.status = a.status;
   p.n_out = a.n_out;

@@ -61,7 +61,8 @@ static_assert(ring_stages(256) >= 4 && ring_stages(kMaxTile) >= 3, "the widest t
 static_assert(8 * (2 * kMaxStages + 4) + 16 <= kBarBytes, "barrier area");
 
 struct BandParams {
-  const void* bias;
+  const void* bias;       // as SparseGemmArgs
+  const void* bias_up;
   void* y;
   int* status;
   int n_out, m_tok, ldy;
@@ -345,20 +346,23 @@ sparse_gemm_band_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_co
         if (row_w + g + 16 < p.n_out) b2 = bias_at(p.bias, row_w + g + 16, p.fmt);
         if (row_w + g + 24 < p.n_out) b3 = bias_at(p.bias, row_w + g + 24, p.fmt);
       }
+      if (EPI == kEpiSwiGLU) load_gate_up_bias(p.bias, p.bias_up, row_w, g, p.n_out, p.fmt, b0, b1, b2, b3);
       // one chunk: activation / SiLU.mul, transpose through the staging tile, 16-byte stores
       auto store_chunk = [&](const uint32_t (&r)[16], int t0) {
         const uint32_t* a = &r[0];
         const uint32_t* b = &r[8];
         __syncwarp();                                 // every lane has read the tile's previous contents
         if (EPI == kEpiSwiGLU) {
-          auto emit = [&](const int of) {
-            stmatrix_x4_trans(stage + st_off, pack16(silu_mul(a[0], b[0]), silu_mul(a[1], b[1]), of),
-                              pack16(silu_mul(a[2], b[2]), silu_mul(a[3], b[3]), of),
-                              pack16(silu_mul(a[4], b[4]), silu_mul(a[5], b[5]), of),
-                              pack16(silu_mul(a[6], b[6]), silu_mul(a[7], b[7]), of));
+          auto emit = [&](auto f, const int of) {
+            stmatrix_x4_trans(stage + st_off, pack16(f(a[0], b[0], b0, b2), f(a[1], b[1], b0, b2), of),
+                              pack16(f(a[2], b[2], b1, b3), f(a[3], b[3], b1, b3), of),
+                              pack16(f(a[4], b[4], b0, b2), f(a[5], b[5], b0, b2), of),
+                              pack16(f(a[6], b[6], b1, b3), f(a[7], b[7], b1, b3), of));
           };
-          if (p.fmt == 1) emit(1);
-          else emit(0);
+          auto plain = [](uint32_t gate, uint32_t up, float, float) { return silu_mul(gate, up); };
+          if (p.bias != nullptr || p.bias_up != nullptr) emit(silu_mul_bias, p.fmt);
+          else if (p.fmt == 1) emit(plain, 1);
+          else emit(plain, 0);
         } else {
           auto emit = [&](auto f, const int of) {
             stmatrix_x4_trans(stage + st_off, pack16(f(a[0], b0), f(a[1], b0), of), pack16(f(a[2], b1), f(a[3], b1), of),
@@ -523,6 +527,7 @@ int launch_band(const SparseGemmArgs& a, int split, int t, cudaStream_t stream) 
   }
   BandParams p;
   p.bias = a.bias;
+  p.bias_up = a.bias_up;
   p.y = a.y;
   p.status = a.status;
   p.n_out = a.n_out;

@@ -48,7 +48,8 @@ struct SmallParams {
   const uint16_t* x;
   const uint16_t* values;
   const uint32_t* meta;
-  const uint16_t* bias;
+  const uint16_t* bias;      // as SparseGemmArgs
+  const uint16_t* bias_up;
   uint16_t* y;
   int m_tok, n_out, K, ldx, ldy;
   int k_tiles128;
@@ -301,6 +302,11 @@ __global__ void __launch_bounds__(kWarps * 32) sparse_gemm_small_m_kernel(const 
       if (SWIGLU) {
         const int f = slab * 16 + r;                      // hidden feature
         if (f < p.n_out / 2) {
+          auto widen = [](uint16_t b) {
+            return BF16 ? __uint_as_float(static_cast<uint32_t>(b) << 16) : __half2float(__ushort_as_half(b));
+          };
+          if (p.bias) s += widen(p.bias[f]);
+          if (p.bias_up) s2 += widen(p.bias_up[f]);
           const float h = (s * __fdividef(1.f, 1.f + __expf(-s))) * s2;
           p.y[static_cast<size_t>(tok) * p.ldy + f] =
               BF16 ? __bfloat16_as_ushort(__float2bfloat16_rn(h)) : __half_as_ushort(__float2half_rn(h));
@@ -382,6 +388,7 @@ int launch_sparse_gemm_small_m(const SparseGemmArgs& a, cudaStream_t stream) {
   p.values = static_cast<const uint16_t*>(a.values);
   p.meta = static_cast<const uint32_t*>(a.meta);
   p.bias = static_cast<const uint16_t*>(a.bias);
+  p.bias_up = static_cast<const uint16_t*>(a.bias_up);
   p.y = static_cast<uint16_t*>(a.y);
   p.m_tok = a.m_tok;
   p.n_out = a.n_out;

