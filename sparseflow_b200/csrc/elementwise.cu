@@ -49,8 +49,8 @@ __global__ void __launch_bounds__(256) silu_mul_vec_kernel(const uint16_t* g, co
   const int c = static_cast<int>(blockIdx.x * 256 + threadIdx.x) * 8;
   if (c >= cols) return;
   for (int r = blockIdx.y; r < rows; r += gridDim.y) {
-    const uint4 gv = __ldg(reinterpret_cast<const uint4*>(g + static_cast<size_t>(r) * ldg + c));
-    const uint4 uv = __ldg(reinterpret_cast<const uint4*>(u + static_cast<size_t>(r) * ldu + c));
+    const uint4 gv = *reinterpret_cast<const uint4*>(g + static_cast<size_t>(r) * ldg + c);
+    const uint4 uv = *reinterpret_cast<const uint4*>(u + static_cast<size_t>(r) * ldu + c);
     uint4 ov;
     ov.x = silu_mul2<BF16>(gv.x, uv.x);
     ov.y = silu_mul2<BF16>(gv.y, uv.y);

@@ -6,6 +6,9 @@
 // kernels launched this way:
 //   * before dependency_wait nothing is read or written but launch parameters; the weights are only PREFETCHED into L2,
 //     which is right whoever wrote them last;
+//   * what a predecessor may have written is read with ordinary loads (or TMA / cp.async) after dependency_wait, never through
+//     the read-only path (__ldg, ld.global.nc, const __restrict__): that is for data nobody writes while the kernel runs, and
+//     this kernel is running while its predecessor writes;
 //   * dependency_trigger comes after dependency_wait, so a kernel that starts early finds everything up to the kernel two
 //     before it complete: at most two kernels of a stream overlap;
 //   * every block executes dependency_wait, so the completion of the kernel implies that of its predecessors.

@@ -154,7 +154,7 @@ struct Row16 {
 };
 __device__ __forceinline__ Row16 load_row16(const PruneParams& p, int r, int k0) {
   const uint4* s = reinterpret_cast<const uint4*>(src_row(p, r) + k0);
-  return Row16{__ldg(s), __ldg(s + 1)};
+  return Row16{s[0], s[1]};
 }
 
 // More than two non-zeros in a group of four (lo, hi), for either of two groups at once.
@@ -260,7 +260,7 @@ __global__ void __launch_bounds__(256) prune_flat_kernel(const __grid_constant__
   if (e >= n) return;
   const uint16_t* s = p.src0 + e;
   if (e + 16 <= n) {
-    const uint4 a = __ldg(reinterpret_cast<const uint4*>(s)), b = __ldg(reinterpret_cast<const uint4*>(s) + 1);
+    const uint4 a = reinterpret_cast<const uint4*>(s)[0], b = reinterpret_cast<const uint4*>(s)[1];
     prune_store16<TIE>(p, lut, a, b, e / 2, e, e / 4);
   } else {
     for (size_t i = e; i < n; i += 4) prune_store4<TIE>(p, lut, *reinterpret_cast<const uint2*>(p.src0 + i), i);
@@ -303,7 +303,7 @@ __global__ void __launch_bounds__(256) validate_flat_kernel(const uint16_t* w, s
   const size_t step = static_cast<size_t>(gridDim.x) * blockDim.x * 16;
   for (size_t e = (blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x) * 16; e < n; e += step) {
     if (e + 16 <= n) {
-      const uint4 a = __ldg(reinterpret_cast<const uint4*>(w + e)), b = __ldg(reinterpret_cast<const uint4*>(w + e) + 1);
+      const uint4 a = reinterpret_cast<const uint4*>(w + e)[0], b = reinterpret_cast<const uint4*>(w + e)[1];
       bad |= not_24(a.x, a.y, a.z, a.w) || not_24(b.x, b.y, b.z, b.w);
     } else {
       for (size_t i = e; i < n; i += 4) {

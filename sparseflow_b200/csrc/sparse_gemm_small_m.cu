@@ -182,7 +182,7 @@ __global__ void __launch_bounds__(kWarps * 32) sparse_gemm_small_m_kernel(const 
 #pragma unroll 4
     for (int i = lane; i < chunks * p.m_tok; i += 32) {
       const int tok = i / chunks, c = i - tok * chunks;
-      const uint4 v = __ldg(reinterpret_cast<const uint4*>(p.x + static_cast<size_t>(tok) * p.ldx + k_lo + c * 8));
+      const uint4 v = *reinterpret_cast<const uint4*>(p.x + static_cast<size_t>(tok) * p.ldx + k_lo + c * 8);
       uint32_t* d = reinterpret_cast<uint32_t*>(xs + ((c >> 2) * p.m_tok + tok) * 4) + (c & 3);
       d[0] = v.x;
       d[4] = v.y;
@@ -209,7 +209,7 @@ __global__ void __launch_bounds__(kWarps * 32) sparse_gemm_small_m_kernel(const 
         const bool ok = tok < p.m_tok && k0 < p.K;
         const uint32_t* xp = reinterpret_cast<const uint32_t*>(p.x + static_cast<size_t>(ok ? tok : 0) * p.ldx + (ok ? k0 : 0) + 2 * t);
 #pragma unroll
-        for (int q = 0; q < 4; ++q) dst[kb][n][q] = ok ? __ldg(xp + 4 * q) : 0u;
+        for (int q = 0; q < 4; ++q) dst[kb][n][q] = ok ? xp[4 * q] : 0u;
       }
     }
   };
