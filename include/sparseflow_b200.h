@@ -305,7 +305,7 @@ SFB200_API int sfb200_blob_read_header(const void* header_host, size_t available
  * CTA-pair kernel, 256-row x 256-token tiles; 1192/1208/1224/1240 = the same with that many tokens and
  * two accumulator sets; 5192/5208/5224/5240 = CTA-pair kernel, 512-row tiles with that many tokens and
  * 128-wide K stages (2192..2240: the same with 64-wide stages); 3032/3064/3128 and 4032/4064/4128 = split-K cluster kernel with 2 or 4
- * K slices and a 32/64/128-token tile; 6000 / 7000 / 9000 / 8000 + t = CTA-pair kernel with a token tile of t (a
+ * K slices and a 32/64/128-token tile (128: only when forced); 6000 / 7000 / 9000 / 8000 + t = CTA-pair kernel with a token tile of t (a
  * multiple of 16 up to 400) and K split over 1 / 2 / 3 / 4 pairs.  No counterpart upstream. */
 SFB200_API int sfb200_debug_force_token_tile(int bn);
 
@@ -314,10 +314,9 @@ SFB200_API int sfb200_debug_force_token_tile(int bn);
  * operand: -1 automatic (the smaller of activations and compressed weight), 0 activations, 1 weights. */
 SFB200_API int sfb200_debug_pair_tuning(int l2_band_mb, int force_order);
 
-/* For Y[M, N] = X[M, K] . W^T (swiglu = 1: the fused gate|up GEMM, N = 2 * I rows) on a GPU with num_sms SMs, in the
- * numbering above; 0 for a non-positive size.  Host-only.  _plan_gemm: the choice among the kernels of fixed tiles;
- * _route_gemm: what a call with nothing forced runs: that choice, one of the 6000 ... 9000 forms where it is faster, or a 512-row pair
- * tile in place of a 256-row one where that is faster at the power limit. */
+/* The variant the library picks on its own for Y[M, N] = X[M, K] . W^T (swiglu = 1: the fused gate|up GEMM,
+ * N = 2 * I rows) on a GPU with num_sms SMs, in the numbering above; 0 for a non-positive size.  Host-only.  Both names
+ * give the same answer. */
 SFB200_API int sfb200_debug_plan_gemm(int M, int N, int K, int swiglu, int num_sms);
 SFB200_API int sfb200_debug_route_gemm(int M, int N, int K, int swiglu, int num_sms);
 

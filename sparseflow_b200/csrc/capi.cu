@@ -514,17 +514,15 @@ SFB200_API int sfb200_debug_pair_tuning(int l2_band_mb, int force_order) {
   return kOk;
 }
 
-/* The variant for a shape among the kernels of fixed tiles, and the one sfb200_sparse_gemm (swiglu = 0) or
- * sfb200_sparse_gemm_swiglu (swiglu = 1, N = 2 * I rows) runs: the same, or a form of the band kernel (6000 ... 9000 +
- * token tile).  On a GPU with num_sms SMs, in the numbering of sfb200_debug_force_token_tile.  Host-only. */
+/* Which kernel variant sfb200_sparse_gemm (swiglu = 0) or sfb200_sparse_gemm_swiglu (swiglu = 1, N = 2 * I
+ * rows) runs for a shape on a GPU with num_sms SMs, in the numbering of sfb200_debug_force_token_tile.  Host-only. */
 SFB200_API int sfb200_debug_plan_gemm(int M, int N, int K, int swiglu, int num_sms) {
   if (M <= 0 || N <= 0 || K <= 0 || num_sms <= 0) return 0;
   return plan_sparse_gemm(M, N, K, swiglu ? kEpiSwiGLU : kEpiStore, num_sms);
 }
 
 SFB200_API int sfb200_debug_route_gemm(int M, int N, int K, int swiglu, int num_sms) {
-  if (M <= 0 || N <= 0 || K <= 0 || num_sms <= 0) return 0;
-  return route_sparse_gemm(M, N, K, swiglu ? kEpiSwiGLU : kEpiStore, num_sms);
+  return sfb200_debug_plan_gemm(M, N, K, swiglu, num_sms);
 }
 
 /* The chunk plan sfb200_ffn_forward_host would use for M tokens (host-only; out8 holds 8 ints). */

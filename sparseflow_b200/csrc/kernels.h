@@ -82,7 +82,7 @@ struct SparseGemmArgs {
 };
 int launch_sparse_gemm(const SparseGemmArgs& a, cudaStream_t stream);
 // CTA-pair (cta_group::2) kernel; launch_sparse_gemm goes straight to it from 4 * kPairMinTokens tokens and weighs it
-// against the single-CTA tiles below that.  force_bn 1192..1256 (256-row tiles), 5192..5240 (512-row tiles, 128-wide
+// against the single-CTA and band tiles below that.  force_bn 1192..1256 (256-row tiles), 5192..5240 (512-row tiles, 128-wide
 // K stages) or 2192..2240 (512-row tiles, 64-wide stages) picks a variant.
 int launch_sparse_gemm_pair(const SparseGemmArgs& a, cudaStream_t stream);
 constexpr int kPairMinTokens = 1024;
@@ -94,9 +94,10 @@ void set_pair_tuning(int l2_band_mb, int force_order);
 int pick_pair_variant(int n_out, int m_tok, int K, int num_sms, int swiglu, double* cost_us = nullptr);
 // The same with a preference for the 512-row tiles, which need less energy.
 int pick_pair_variant_sustained(int n_out, int m_tok, int K, int num_sms, int swiglu);
-// The kernel variant for a shape among the kernels of fixed tiles, in the numbering of
+// The kernel variant launch_sparse_gemm runs for a 16-bit result when nothing is forced, in the numbering of
 // SparseGemmArgs::force_bn: 8 decode kernel; 32..256 single-CTA kernel with that token tile; 1192..1256 / 5192..5240
-// CTA-pair kernel; 3000 + tile / 4000 + tile split-K cluster kernel with 2 / 4 K slices.  Host-only.
+// CTA-pair kernel; 3000 + tile / 4000 + tile split-K cluster kernel with 2 / 4 K slices; 6000 / 7000 / 9000 / 8000 + tile band
+// kernel with K split over 1 / 2 / 3 / 4 pairs.  Host-only.
 int plan_sparse_gemm(int m_tok, int n_out, int K, int epi, int num_sms);
 // The exchange step (reduction + all-gather) of the row-parallel GEMM in one launch per rank, cross-GPU ordering
 // included.  mode 3: src = LOCAL receive slots [tp][slot_rows, cols] (slots_f32 = 0: 16-bit of the output type, 1: float, 2: fp16 whatever the output type) that the ranks' GEMM
@@ -121,8 +122,8 @@ int launch_exchange(int mode, const void* src, void* mc_dst, void* const* peer_d
                     int* status, cudaStream_t stream, const ExchangePush* push = nullptr);
 
 // Split-K variant of the single-CTA kernel: a cluster of `split` (2 or 4) CTAs shares one output tile,
-// each streaming a slice of K; partial tiles are reduced through distributed shared memory.  Chosen by
-// launch_sparse_gemm when splitk_factor() > 1 (too few row tiles to occupy the SMs).  kEpiStore only.
+// each streaming a slice of K; partial tiles are reduced through distributed shared memory.  For up to 64 tokens when
+// splitk_factor() > 1 (too few row tiles to occupy the SMs); a 128-token tile runs when forced only.  kEpiStore only.
 int launch_sparse_gemm_splitk(const SparseGemmArgs& a, int split, cudaStream_t stream);
 int splitk_factor(int m_tok, int n_out, int K, int num_sms);
 int splitk_token_tile(int m_tok);
@@ -134,17 +135,15 @@ int launch_sparse_gemm_band(const SparseGemmArgs& a, cudaStream_t stream);
 int pick_band_variant(int m_tok, int n_out, int K, int num_sms, double* cost_us = nullptr);
 // Whether a split-1 form cuts left-over tiles into token slices for a shape.
 bool band_has_slices(int m_tok, int n_out, int num_sms, int variant);
-// What launch_sparse_gemm runs for a 16-bit result when nothing is forced: the band form where it is the faster one, a
-// 512-row pair tile where that needs less energy, else plan_sparse_gemm's choice among the fixed tiles.  Host-only.
-int route_sparse_gemm(int m_tok, int n_out, int K, int epi, int num_sms);
 
 // ---- small-M (decode) sparse GEMM ----------------------------------------------------------
-// Supports M <= 32 tokens; chosen by launch_sparse_gemm for m_tok <= kSmallMMaxTokens (force_bn == 8 forces it).
+// Supports M <= 32 tokens; plan_sparse_gemm chooses it for up to 8 (force_bn == 8 forces it).
 int launch_sparse_gemm_small_m(const SparseGemmArgs& a, cudaStream_t stream);
 // Where the split-K cluster kernel applies too (few row tiles): whether this one is the faster, i.e. it has no second, partly
 // filled round of 16-row slabs -- at most one slab per SM, or two blocks per SM with the X cache in shared memory.
 bool small_m_beats_splitk(int m_tok, int n_out, int K, int num_sms);
-constexpr int kSmallMMaxTokens = 4;   // from 5 tokens the tcgen05 kernel with a 32-token tile is faster (measured)
+// From 5 tokens the tcgen05 kernel with a 32-token tile is faster (measured); on few row tiles small_m_beats_splitk decides.
+constexpr int kSmallMMaxTokens = 4;
 
 // ---- elementwise -----------------------------------------------------------------------------
 // out[m, i] = silu(gu[m, i]) * gu[m, I + i]   (unfused variant, gate|up concatenated along columns)

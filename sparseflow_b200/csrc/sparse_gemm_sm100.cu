@@ -373,16 +373,16 @@ int launch_cfg(const SparseGemmArgs& a, cudaStream_t stream) {
   return launch_dependent(sparse_gemm_kernel<C>, grid, 192, C::SMEM_BYTES, 0, stream, tmA, tmB, tmD, p);
 }
 
-// Kernel / token-tile choice from 129 tokens up: the cheapest, by estimated time, of the single-CTA tiles and the
-// CTA-pair tiles.  Up to about a thousand tokens every candidate is bound by operand traffic, not by the tensor pipe,
-// and what decides is how many passes ("waves") the tile count needs on the available SMs (or SM pairs):
+// The cheapest, by estimated time, of the single-CTA tiles and the CTA-pair tiles, from 161 to 4095 tokens.  Up to about
+// a thousand tokens every candidate is bound by operand traffic, not by the tensor pipe, and what decides is how many passes
+// ("waves") the tile count needs on the available SMs (or SM pairs):
 //   single-CTA tile of bn tokens: waves x 64-wide K steps x step time + 8.5 us, where a step moves 9 KiB (values +
 //     metadata) + bn x 128 B (tokens), an SM sustains about 145 GB/s of operand traffic and all SMs together about
 //     19.5 TB/s out of L2 (17 TB/s for the 256-token tile, whose ring is only four stages deep);
 //   CTA-pair tiles: pick_pair_variant's estimate.
 // Measured on B200 (variants timed as CUDA graphs against this model): 22016 x 4096 at 1024 tokens 112 -> 88 us with the
-// 256 x 208 pair tile; 4096 x 11008 at 1024 tokens stays with the single-CTA 256-token tile (32 row tiles x 4 = 128 tiles
-// = one wave on 148 SMs, 59.6 us, against two waves of pair tiles, 66 us).
+// 256 x 208 pair tile; 4096 x 11008 at 1024 tokens 46 us with the 256 x 256 pair tile (64 tiles, one wave of pairs) against
+// 59.6 us with the single-CTA 256-token tile.
 int pick_mid_variant(int n_out, int m_tok, int K, int num_sms, int swiglu, double* cost_us = nullptr) {
   const double k64 = (K + 63) / 64;
   const long mb = (n_out + 127) / 128;
@@ -422,36 +422,6 @@ int dispatch_bn(const SparseGemmArgs& a, cudaStream_t stream) {
   }
 }
 
-}  // namespace
-
-int plan_sparse_gemm(int m_tok, int n_out, int K, int epi, int num_sms) {
-  // few row tiles (the weight has fewer 128-row tiles than half the SMs) and fewer tokens than the
-  // prefill kernel wants: split K over a cluster so that the weight is streamed by (nearly) every SM
-  const int split = (epi == kEpiStore && m_tok < kPairMinTokens) ? splitk_factor(m_tok, n_out, K, num_sms) : 1;
-  // decode-sized token counts: bandwidth kernel on warp-level mma.sp; measured against the split-K
-  // kernel it only wins at 1-2 tokens when both apply
-  if (m_tok <= kSmallMMaxTokens && (split == 1 || m_tok <= 2)) return 8;
-  if (m_tok >= 4 * kPairMinTokens) return pick_pair_variant(n_out, m_tok, K, num_sms, epi == kEpiSwiGLU);   // prefill proper: pair tiles
-  if (m_tok > 64 && m_tok <= 128) {
-    // 65..128 tokens: one 128-token tile per row tile, two 64-token tiles, or split K.  A 128-wide stage of the
-    // 128-token tile holds 50 KB and is feed-bound (~430 ns), of the 64-token tile 34 KB (~268 ns); what decides is
-    // again the number of passes over the SMs.  (Measured: 8192 x 8192 at 128 tokens 27.9 -> 20.5 us with two
-    // 64-token tiles; 22016 x 4096 31.6 -> 28.9 us; 11008 x 4096 and 28672 x 4096 stay with the 128-token tile.)
-    const long mb = (n_out + 127) / 128;
-    const double k128 = (K + 127) / 128;
-    auto waves = [&](long tiles) { return static_cast<double>((tiles + num_sms - 1) / num_sms); };
-    const double c128 = waves(mb) * k128 * 430e-9 + 4e-6;
-    const double c64 = waves(2 * mb) * k128 * 268e-9 + 4e-6;
-    const double csplit = split > 1 ? (k128 / split) * 385e-9 + 10e-6 : 1e30;
-    if (epi == kEpiStore && csplit < c128 && csplit < c64) return (split == 4 ? 4000 : 3000) + 128;
-    return c64 < c128 ? 64 : 128;
-  }
-  if (split > 1) return (split == 4 ? 4000 : 3000) + splitk_token_tile(m_tok);
-  if (m_tok <= 32) return 32;
-  if (m_tok <= 64) return 64;
-  return pick_mid_variant(n_out, m_tok, K, num_sms, epi == kEpiSwiGLU);
-}
-
 // Estimated time in us of the single-CTA 64-token tiles: a 128-wide K step costs 0.215 us, the weights stream at 6.6 TB/s and
 // 0.45 of the shorter of the two adds (11008 x 4096 at 64 tokens 13.5 us, 6000 x 3072 at 72 tokens 8.7 us, 8192 x 8192 at 128
 // tokens 22.0 us measured).
@@ -461,31 +431,42 @@ double tile64_cost(int m_tok, int n_out, int K, int num_sms) {
   return 2.6 + (comp > hbm ? comp + 0.45 * hbm : hbm + 0.45 * comp);
 }
 
-// From 33 to 1023 tokens the band kernel (sparse_gemm_sm100_band.cu) is weighed against the fixed tiles by estimated time.
-//   33-64 tokens: only where the plan would split K in two (38-74 row tiles): 8192 x 8192 at 64 tokens 20.8 -> 17.8 us, 6000 x
-//     3072 12.6 -> 9.1 us (the 64-token tile);
-//   65-128: against the 64-token tiles (6000 x 3072 at 72 tokens 8.7 against 10.1 us, 22016 x 4096 29.2 against 26.2);
-//   129-160: the band kernel outright, 1.1-1.9 x the fixed choice on every shape measured (4096 x 11008 at 150 tokens 34.6 ->
-//     18.5 us, 22016 x 4096 32.8 -> 25.2 us);
-//   above: the lower estimate (300 tokens: 4096 x 11008 34.4 -> 21.6 us, 22016 x 4096 42.1 -> 34.8 us; 520 tokens: 8192 x 8192
-//     55.5 -> 42.0 us; at 700-1000 tokens the two meet).
-int route_sparse_gemm(int m_tok, int n_out, int K, int epi, int num_sms) {
-  const int fixed = plan_sparse_gemm(m_tok, n_out, K, epi, num_sms);
-  if (m_tok >= kPairMinTokens && fixed >= 1192 && fixed <= 1240)
-    return pick_pair_variant_sustained(n_out, m_tok, K, num_sms, epi == kEpiSwiGLU);
-  if (m_tok <= 8 && epi == kEpiStore) {
-    // decode on few row tiles: slab kernel or split K.  Measured at 1 / 2 / 8 tokens, slabs against split K: 2048 x 2048 2.8 /
-    // 3.0 / 4.0 against 4.5 us; 4096 x 4096 5.3 / 6.0 / 8.4 against 6.8-7.2; 4096 x 11008 11.0 / 13.6 / 20.1 against 11.8;
-    // 4096 x 14336 15.3 / 16.6 / 24.9 against 13.9; 8192 x 8192 15.3 / 17.0 / 21.8 against 15.8.
-    const int split = splitk_factor(m_tok, n_out, K, num_sms);
-    if (split > 1) return small_m_beats_splitk(m_tok, n_out, K, num_sms) ? 8 : (split == 4 ? 4000 : 3000) + splitk_token_tile(m_tok);
+}  // namespace
+
+// What launch_sparse_gemm runs.  By token count:
+//   1-8, few row tiles (the weight has fewer 128-row tiles than half the SMs, so splitk_factor > 1): slab kernel or split K,
+//     small_m_beats_splitk;
+//   1-4 otherwise: the slab kernel;
+//   to 32: the 32-token tile, or split K on few row tiles;
+//   33-64: the 64-token tile, four K slices where there are at most a quarter as many row tiles as SMs, the band kernel
+//     (sparse_gemm_sm100_band.cu) where two slices would fit (38-74 row tiles): 8192 x 8192 at 64 tokens 20.8 us split in two,
+//     17.8 us;
+//   65-128: 64-token tiles or band kernel by estimated time (6000 x 3072 at 72 tokens 8.7 against 10.1 us, 22016 x 4096 29.2
+//     against 26.2);
+//   129-160: the band kernel outright, 1.1-1.9 x the fixed tiles on every shape measured (bursts: 4096 x 11008 at 150 tokens 34.6
+//     -> 17.0 us, 22016 x 4096 32.8 -> 25.2 us);
+//   161-1023: band kernel or fixed tiles by estimated time (bursts, 300 tokens: 4096 x 11008 34.4 -> 21.6 us, 22016 x 4096 42.1 ->
+//     32.6 us; steady, 520 tokens: 8192 x 8192 55.5 -> 42.0 us; at 700-1000 tokens the two meet);
+//   from 1024: pair or single-CTA tiles, to 4095 by estimated time, above that pair tiles; a 512-row tile in place of a
+//     256-row one with two accumulator sets where pick_pair_variant_sustained prefers it.
+int plan_sparse_gemm(int m_tok, int n_out, int K, int epi, int num_sms) {
+  const int swiglu = epi == kEpiSwiGLU;
+  if (m_tok >= kPairMinTokens) {
+    const int v = m_tok >= 4 * kPairMinTokens ? pick_pair_variant(n_out, m_tok, K, num_sms, swiglu)
+                                              : pick_mid_variant(n_out, m_tok, K, num_sms, swiglu);
+    return v >= 1192 && v <= 1240 ? pick_pair_variant_sustained(n_out, m_tok, K, num_sms, swiglu) : v;
   }
-  if (m_tok >= kPairMinTokens || m_tok <= 32 || (m_tok <= 64 && (fixed < 3000 || fixed >= 4000))) return fixed;
+  const int split = epi == kEpiStore ? splitk_factor(m_tok, n_out, K, num_sms) : 1;
+  const int by_split = (split == 4 ? 4000 : 3000) + splitk_token_tile(m_tok);
+  if (m_tok <= 8 && split > 1) return small_m_beats_splitk(m_tok, n_out, K, num_sms) ? 8 : by_split;
+  if (m_tok <= kSmallMMaxTokens) return 8;
+  if (m_tok <= 32) return split > 1 ? by_split : 32;
+  if (m_tok <= 64 && split != 2) return split == 4 ? by_split : 64;
   double band_us = 0.0, fixed_us = 0.0;
   const int band = pick_band_variant(m_tok, n_out, K, num_sms, &band_us);
   if (m_tok <= 128) return tile64_cost(m_tok, n_out, K, num_sms) < band_us ? 64 : band;
   if (m_tok <= 160) return band;
-  pick_mid_variant(n_out, m_tok, K, num_sms, epi == kEpiSwiGLU, &fixed_us);
+  const int fixed = pick_mid_variant(n_out, m_tok, K, num_sms, swiglu, &fixed_us);
   // The same tile as the fixed kernel's, with no left-over tiles to slice, has nothing to gain (2-4 % slower).  Above 800
   // tokens the estimate is trusted by a wider margin: there the tiles with a single accumulator set fall behind it
   // (8192 x 28672 at 1000 tokens estimated 0.95, measured 1.17 of the fixed tile).
@@ -508,7 +489,7 @@ int launch_sparse_gemm(const SparseGemmArgs& a, cudaStream_t stream) {
       b.force_bn = pick_pair_variant(a.n_out, a.m_tok, a.K, a.num_sms, 0);
     return launch_sparse_gemm_pair(b, stream);
   }
-  if (b.force_bn == 0) b.force_bn = route_sparse_gemm(a.m_tok, a.n_out, a.K, a.epi, a.num_sms);
+  if (b.force_bn == 0) b.force_bn = plan_sparse_gemm(a.m_tok, a.n_out, a.K, a.epi, a.num_sms);
   const int v = b.force_bn;
   if (v == 8) return launch_sparse_gemm_small_m(b, stream);
   if (v >= 6000) return launch_sparse_gemm_band(b, stream);

@@ -252,29 +252,30 @@ def test_kernel_plan_per_shape():
     """Which kernel the dispatcher runs for the benchmark shapes on a 148-SM GPU (host-only planning call)."""
     from sparseflow_b200 import _lib
     plan = lambda M, N, K, sw=0: _lib.lib().sfb200_debug_plan_gemm(M, N, K, sw, 148)
-    # decode: many row tiles -> warp-level kernel up to 4 tokens; few row tiles -> it keeps only 1-2 tokens
+    # decode: many row tiles -> warp-level kernel up to 4 tokens; few row tiles -> it or split K, up to 8 tokens
     assert plan(1, 28672, 4096) == 8 and plan(4, 28672, 4096) == 8 and plan(4, 22016, 4096, 1) == 8
     assert plan(5, 28672, 4096) == 32 and plan(8, 22016, 4096, 1) == 32
-    assert plan(2, 4096, 14336) == 8 and plan(4, 4096, 14336) == 4032
-    # few row tiles, below the prefill threshold: split-K over a cluster, 4 slices for 32 tiles, 2 for 64
-    assert plan(32, 4096, 11008) == 4032 and plan(64, 4096, 11008) == 4064 and plan(128, 4096, 11008) == 4128
-    assert plan(16, 8192, 8192) == 3032 and plan(64, 8192, 8192) == 3064
-    # 65..128 tokens: two 64-token tiles where they need no more passes over the SMs than one 128-token tile
-    assert plan(128, 8192, 8192) == 64 and plan(128, 4096, 4096) == 64 and plan(128, 22016, 4096) == 64
-    assert plan(128, 11008, 4096) == 128 and plan(100, 28672, 4096) == 128
+    assert plan(1, 4096, 11008) == 8 and plan(2, 4096, 11008) == 4032 and plan(1, 4096, 14336) == 4032
+    assert plan(8, 2048, 2048) == 8 and plan(9, 2048, 2048) == 4032 and plan(8, 4096, 4096) == 4032
+    # few row tiles, up to 64 tokens: split-K over a cluster, 4 slices for 32 tiles, 2 for 64 (to 32 tokens; then CTA pairs, K split)
+    assert plan(32, 4096, 11008) == 4032 and plan(64, 4096, 11008) == 4064
+    assert plan(16, 8192, 8192) == 3032 and plan(33, 8192, 8192) == 7048 and plan(64, 8192, 8192) == 7064
+    # 65..128 tokens: 64-token tiles or CTA pairs with a run-time token tile, by estimated time
+    assert plan(128, 8192, 8192) == 7128 and plan(128, 4096, 4096) == 9128 and plan(128, 22016, 4096) == 6128
+    assert plan(72, 6000, 3072) == 64 and plan(72, 22016, 4096) == 6080 and plan(100, 28672, 4096) == 6112
     assert plan(32, 512, 256) == 32                   # too little K to split (< 4 metadata tiles per slice)
     # many row tiles, up to 128 tokens: single-CTA kernel with the smallest covering token tile
-    assert plan(9, 22016, 4096) == 32 and plan(33, 22016, 4096) == 64 and plan(100, 11008, 4096) == 128
+    assert plan(9, 22016, 4096) == 32 and plan(33, 22016, 4096) == 64
     assert plan(64, 22016, 4096, 1) == 64             # the SwiGLU epilogue has no split-K form
-    # from 129 tokens: the cheapest of single-CTA tiles and CTA-pair tiles by estimated time (passes over the SMs)
-    assert plan(512, 14336, 4096) == 1192 and plan(512, 22016, 4096, 1) == 1192 and plan(1024, 22016, 4096, 1) == 5208
-    assert plan(256, 4096, 4096) == 128 and plan(512, 4096, 14336) == 128 and plan(768, 4096, 11008) == 1192
+    # 129..1023 tokens: pairs with a run-time token tile, K split where row tiles are few, or fixed tiles, by estimated time
+    assert plan(150, 4096, 11008) == 9160 and plan(150, 22016, 4096, 1) == 6160 and plan(300, 22016, 4096, 1) == 6304
+    assert plan(300, 4096, 11008) == 7160 and plan(512, 28672, 4096, 1) == 6256 and plan(512, 4096, 14336) == 7256
+    assert plan(520, 8192, 8192) == 6272 and plan(512, 8192, 8192) == 1256 and plan(256, 14336, 4096) == 1256
     # the 256 x 256 pair tile where it covers the output in ONE pass over the 74 SM pairs and the others need two
-    assert plan(1024, 4096, 4096) == 1256 and plan(1024, 4096, 11008) == 1256 and plan(512, 8192, 8192) == 1256
-    assert plan(256, 14336, 4096) == 1256
+    assert plan(1024, 4096, 4096) == 1256 and plan(1024, 4096, 11008) == 1256 and plan(1024, 22016, 4096, 1) == 5208
     # prefill: 256-row tiles with two accumulator sets where K is short (the drain hides behind the next tile), 512-row
     # tiles (the token tile is read by two row sets) where K is long or the passes over the SM pairs come out fewer
-    assert plan(4096, 22016, 4096, 1) == 1240 and plan(4096, 4096, 4096) == 1240 and plan(2048, 22016, 4096, 1) == 5208
+    assert plan(4096, 22016, 4096, 1) == 5240 and plan(2048, 22016, 4096, 1) == 5208
     assert plan(4096, 4096, 11008) == 5240 and plan(4096, 4096, 14336) == 5240 and plan(2048, 4096, 11008) == 5240
     assert plan(8192, 57344, 8192, 1) == 5240 and plan(8192, 8192, 28672) == 5224 and plan(16384, 8192, 8192) == 5240
     assert plan(0, 4096, 4096) == 0
@@ -282,13 +283,14 @@ def test_kernel_plan_per_shape():
 
 def test_kernel_plan_is_always_a_known_variant():
     """Every shape gets a variant the dispatcher knows, and the families keep to their token ranges: decode kernel up to
-    4 tokens, split-K cluster kernel up to 128, 512-row pair tiles from 1024."""
+    8 tokens, split-K cluster kernel up to 64, band kernel from 33 to 1023, 512-row pair tiles from 1024."""
     from sparseflow_b200 import _lib
     plan = _lib.lib().sfb200_debug_plan_gemm
     single = {32, 64, 128, 192, 256}
     pair = {1192, 1208, 1224, 1240, 1256}
     pair512 = {5192, 5208, 5224, 5240}
-    splitk = {3032, 3064, 3128, 4032, 4064, 4128}
+    splitk = {3032, 3064, 4032, 4064}
+    band = {form + t for form in (6000, 7000, 8000, 9000) for t in range(16, 401, 16)}
     for sms in (148, 132, 64):
         for (N, K) in ((4096, 4096), (22016, 4096), (4096, 11008), (28672, 4096), (4096, 14336), (8192, 8192), (57344, 8192),
                        (8192, 28672), (1024, 1024), (512, 256), (5504, 4096), (4096, 2752)):
@@ -298,11 +300,13 @@ def test_kernel_plan_is_always_a_known_variant():
                     if sw and N % 32:
                         continue
                     v = plan(M, N, K, sw, sms)
-                    assert v == 8 or v in single | pair | pair512 | splitk, (M, N, K, sw, sms, v)
+                    assert v == 8 or v in single | pair | pair512 | splitk | band, (M, N, K, sw, sms, v)
                     if v == 8:
-                        assert M <= 4
+                        assert M <= 4 or (M <= 8 and sw == 0)
                     if v in splitk:
-                        assert M <= 128 and sw == 0
+                        assert M <= 64 and sw == 0
+                    if v in band:
+                        assert 33 <= M <= 1023
                     if v in pair512:
                         assert M >= 1024
                     if M >= 4096:

@@ -312,4 +312,24 @@ def test_random_shapes_through_the_dispatcher():
         rel = ((y - ref).abs() / torch.maximum(ref.abs(), floor)).max().item()
         assert y.shape == (M, N) and rel <= REL_TOL, (M, N, K, rel)
     assert ops.device_status() == 0
-    assert len(seen) >= 6, seen        # decode, single-CTA tiles, split-K and pair variants were all exercised
+    # decode, single-CTA tiles, split-K, pair tiles, band tiles without and with split K were all exercised
+    families = {"decode" if v == 8 else "single" if v < 1000 else "pair" if v < 3000 or 5000 <= v < 6000 else
+                "split K" if v < 5000 else "band" if v < 7000 else "band, split K" for v in seen}
+    assert len(families) == 6, seen
+
+
+# both sides of every token count at which the dispatcher changes its candidates
+@pytest.mark.parametrize("M", [1, 4, 5, 8, 9, 32, 33, 64, 65, 128, 129, 160, 161, 800, 801, 1023, 1024])
+@pytest.mark.parametrize("N,K,swiglu", [(392, 1088, 0), (2048, 2048, 0), (4736, 1024, 0), (8704, 1216, 0), (416, 1088, 1), (8192, 1024, 1)])
+def test_dispatch_boundaries(M, N, K, swiglu):
+    """Nothing forced: whatever the dispatcher picks, in both epilogues, against an fp32 matmul on the decompressed weight."""
+    g = torch.Generator(device="cuda").manual_seed(M + N)
+    x = torch.randn(M, K, generator=g, device="cuda").to(torch.bfloat16)
+    ws = [(torch.randn(N // (1 + swiglu), K, generator=g, device="cuda") * 0.05).to(torch.bfloat16) for _ in range(1 + swiglu)]
+    cws = [ops.compress_weight(w) for w in ws]
+    y = (ops.sparse_gemm_swiglu(x, ops.compress_gate_up(*ws)) if swiglu else ops.sparse_gemm(x, cws[0])).float()
+    assert ops.device_status() == 0
+    refs = [x.float() @ ops.decompress_24(cw).float().t() for cw in cws]
+    ref = torch.nn.functional.silu(refs[0]) * refs[1] if swiglu else refs[0]
+    floor = 1e-2 * ref.pow(2).mean().sqrt()
+    assert ((y - ref).abs() / torch.maximum(ref.abs(), floor)).max().item() <= REL_TOL
