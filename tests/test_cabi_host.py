@@ -281,6 +281,22 @@ def test_kernel_plan_per_shape():
     assert plan(0, 4096, 4096) == 0
 
 
+def test_wide_pair_tiles_only_where_they_are_the_faster_ones():
+    """The preference for 512-row tiles at the power limit: long K and one pass or a tall weight.  The others ran up to 20 % slower on
+    them under steady load (5248 x 1216 at 4726 tokens 33 -> 40 us, 4032 x 9664 at 2662 tokens 105 -> 125 us)."""
+    from sparseflow_b200 import _lib
+    plan = lambda M, N, K, sw=0: _lib.lib().sfb200_debug_plan_gemm(M, N, K, sw, 148)
+    # gate|up of short K, of few rows, of more tokens than half the rows
+    assert plan(4726, 5248, 1216, 1) == 1240 and plan(5570, 7168, 1344, 1) == 1224 and plan(7694, 13600, 1088, 1) == 1240
+    assert plan(2662, 4032, 9664, 1) == 1208 and plan(3575, 3392, 5376, 1) == 1240 and plan(4691, 7616, 3072, 1) == 1224
+    # store epilogue: few rows over several passes, short K
+    assert plan(3578, 2976, 10752) == 1208 and plan(6246, 2784, 7744) == 1192 and plan(1401, 3360, 2752) == 1192
+    assert plan(4096, 4096, 4096) == 1240 and plan(8010, 4736, 4160) == 1240
+    # where they are faster
+    assert plan(4096, 22016, 4096, 1) == 5240 and plan(8192, 22016, 4096, 1) == 5240 and plan(1553, 29568, 5760, 1) == 5224
+    assert plan(1500, 4096, 4096) == 5192 and plan(3000, 11008, 4096) == 5240 and plan(1383, 10080, 5120) == 5208
+
+
 def test_kernel_plan_is_always_a_known_variant():
     """Every shape gets a variant the dispatcher knows, and the families keep to their token ranges: decode kernel up to
     8 tokens, split-K cluster kernel up to 64, band kernel from 33 to 1023, 512-row pair tiles from 1024."""
