@@ -710,10 +710,10 @@ int pick_pair_variant(int n_out, int m_tok, int K, int num_sms, int swiglu, doub
 // fewer bytes through shared memory and 31 % fewer through L2 per flop than a 256-row one.  So a 512-row tile is taken up to
 // an estimate 6 % above the best on the shapes where that measured faster: long K (the 512-row tile has one accumulator set, its
 // drain is not hidden and weighs more the shorter K is) and either one pass over the pairs, store epilogue, or a weight with
-// many more rows than columns and at least twice as many as there are tokens; the SiLU.mul epilogue wants more of both.
+// many more rows than columns and than there are tokens; the SiLU.mul epilogue wants more of both.
 // Steady load, 512-row against 256-row, on the 240 shapes of a sweep where the two choices differ (1024-8192 tokens, K 1024-12288): inside
-// these lines 0.976 on average, worst 1.04 (store: 30 of 88 shapes, 10560 x 4032 at 1267 tokens 64.1 -> 60.7 us; SiLU.mul: 9 of 152, 22016 x
-// 4096 at 4096 tokens 342 -> 333 us); outside them 1.02 (store, worst 2976 x 10752 at 3578 tokens 116 -> 134 us) and 1.06 (SiLU.mul, worst
+// these lines 0.976 on average, worst 1.04 (store: 37 of 88 shapes, 10560 x 4032 at 1267 tokens 64.1 -> 60.7 us; SiLU.mul: 9 of 152, 22016 x
+// 4096 at 4096 tokens 342 -> 333 us); outside them 1.03 (store, worst 2976 x 10752 at 3578 tokens 116 -> 134 us) and 1.06 (SiLU.mul, worst
 // 4032 x 9664 at 2662 tokens 105 -> 125 us, 5248 x 1216 at 4726 tokens 33 -> 40 us), where the estimates alone decide.
 int pick_pair_variant_sustained(int n_out, int m_tok, int K, int num_sms, int swiglu) {
   const int pairs = num_sms / 2 > 0 ? num_sms / 2 : 1;
@@ -721,7 +721,7 @@ int pick_pair_variant_sustained(int n_out, int m_tok, int K, int num_sms, int sw
   if (wide < 5000) return wide;
   const int bn = wide - 5000;
   const long tiles = static_cast<long>((n_out + 511) / 512) * ((m_tok + bn - 1) / bn);
-  const bool tall = n_out >= (swiglu ? 4 : 2) * static_cast<long>(K) && n_out >= 2l * m_tok;
+  const bool tall = swiglu ? n_out >= 4l * K && n_out >= 2l * m_tok : 2l * n_out >= 3l * K && 3l * n_out >= 5l * m_tok;
   if (K >= (swiglu ? 4096 : 3328) && (tall || (!swiglu && tiles <= pairs))) return wide;
   return pick_pair_variant_impl(n_out, m_tok, K, pairs, swiglu, nullptr);
 }
