@@ -373,7 +373,7 @@ int launch_cfg(const SparseGemmArgs& a, cudaStream_t stream) {
   return launch_dependent(sparse_gemm_kernel<C>, grid, 192, C::SMEM_BYTES, 0, stream, tmA, tmB, tmD, p);
 }
 
-// The cheapest, by estimated time, of the single-CTA tiles and the CTA-pair tiles, from 161 to 4095 tokens.  Up to about
+// The cheapest, by estimated time, of the single-CTA tiles and the CTA-pair tiles, from 129 to 4095 tokens.  Up to about
 // a thousand tokens every candidate is bound by operand traffic, not by the tensor pipe, and what decides is how many passes
 // ("waves") the tile count needs on the available SMs (or SM pairs):
 //   single-CTA tile of bn tokens: waves x 64-wide K steps x step time + 8.5 us, where a step moves 9 KiB (values +
@@ -443,10 +443,9 @@ double tile64_cost(int m_tok, int n_out, int K, int num_sms) {
 //     17.8 us;
 //   65-128: 64-token tiles or band kernel by estimated time (6000 x 3072 at 72 tokens 8.7 against 10.1 us, 22016 x 4096 29.2
 //     against 26.2);
-//   129-160: the band kernel outright, 1.1-1.9 x the fixed tiles on every shape measured (bursts: 4096 x 11008 at 150 tokens 34.6
-//     -> 17.0 us, 22016 x 4096 32.8 -> 25.2 us);
-//   161-1023: band kernel or fixed tiles by estimated time (bursts, 300 tokens: 4096 x 11008 34.4 -> 21.6 us, 22016 x 4096 42.1 ->
-//     32.6 us; steady, 520 tokens: 8192 x 8192 55.5 -> 42.0 us; at 700-1000 tokens the two meet);
+//   129-1023: band kernel or fixed tiles by estimated time (bursts: 4096 x 11008 at 150 / 300 tokens 34.6 / 34.4 -> 17.0 / 21.6 us,
+//     22016 x 4096 32.8 / 42.1 -> 25.2 / 32.6 us; steady: 8192 x 8192 at 520 tokens 55.5 -> 42.0 us; at 700-1000 tokens and on small
+//     shapes the two meet).  On 400 random shapes (256-24000 rows, K 512-12288) the choice averages 1.01 of the faster of the two;
 //   from 1024: pair or single-CTA tiles, to 4095 by estimated time, above that pair tiles; a 512-row tile in place of a
 //     256-row one with two accumulator sets where pick_pair_variant_sustained prefers it.
 int plan_sparse_gemm(int m_tok, int n_out, int K, int epi, int num_sms) {
@@ -465,13 +464,18 @@ int plan_sparse_gemm(int m_tok, int n_out, int K, int epi, int num_sms) {
   double band_us = 0.0, fixed_us = 0.0;
   const int band = pick_band_variant(m_tok, n_out, K, num_sms, &band_us);
   if (m_tok <= 128) return tile64_cost(m_tok, n_out, K, num_sms) < band_us ? 64 : band;
-  if (m_tok <= 160) return band;
   const int fixed = pick_mid_variant(n_out, m_tok, K, num_sms, swiglu, &fixed_us);
+  // Those estimates carry 8.5 us outside the K loop, to compare with each other.  Measured as dependent launches it is 3.7 us for the
+  // single-CTA tiles (median of 204 shapes; 4.2 where they meet the band kernel) and, at short K, 5.6 us for the pair tiles (126 shapes);
+  // with 8.5 the band kernel was taken on small shapes where it is the slower one (2240 x 768 at 850 tokens 7.5 against 5.9 us, 8000 x 512 at
+  // 239 tokens 6.8 against 5.3, 9536 x 832 with SiLU.mul at 630 tokens 11.9 against 10.8).
+  if (fixed < 256) fixed_us -= 8.5 - 4.2;
+  else if (K <= 1408) fixed_us -= 8.5 - 5.6;
   // The same tile as the fixed kernel's, with no left-over tiles to slice, has nothing to gain (2-4 % slower).  Above 800
   // tokens the estimate is trusted by a wider margin: there the tiles with a single accumulator set fall behind it
   // (8192 x 28672 at 1000 tokens estimated 0.95, measured 1.17 of the fixed tile).
   if (band % 1000 == fixed % 1000 && fixed >= 1000 && fixed < 3000 && !band_has_slices(m_tok, n_out, num_sms, band)) return fixed;
-  return band_us < (m_tok > 800 ? 0.8 : 1.0) * fixed_us ? band : fixed;
+  return band_us < (m_tok > 800 ? 0.9 : 1.0) * fixed_us ? band : fixed;
 }
 
 int launch_sparse_gemm(const SparseGemmArgs& a, cudaStream_t stream) {

@@ -297,6 +297,16 @@ def test_wide_pair_tiles_only_where_they_are_the_faster_ones():
     assert plan(1500, 4096, 4096) == 5192 and plan(3000, 11008, 4096) == 5240 and plan(1383, 10080, 5120) == 5208
 
 
+def test_small_shapes_keep_the_fixed_tiles():
+    """129-1023 tokens, little K: the fixed tiles are the faster ones (2240 x 768 at 850 tokens 5.9 against 7.5 us, 8000 x 512 at 239
+    tokens 5.3 against 6.8 us), but for a handful of tiles the band kernel is (320 x 704 at 160 tokens 4.3 against 5.8 us)."""
+    from sparseflow_b200 import _lib
+    plan = lambda M, N, K, sw=0: _lib.lib().sfb200_debug_plan_gemm(M, N, K, sw, 148)
+    assert plan(850, 2240, 768) == 128 and plan(461, 4448, 768) == 128 and plan(239, 8000, 512) == 128
+    assert plan(623, 2880, 1280) == 128 and plan(133, 7872, 832) == 128 and plan(630, 9536, 832, 1) == 1224
+    assert plan(160, 320, 704, 1) == 6064 and plan(832, 5152, 2944) == 6208 and plan(158, 15232, 4992, 1) == 6160
+
+
 def test_kernel_plan_is_always_a_known_variant():
     """Every shape gets a variant the dispatcher knows, and the families keep to their token ranges: decode kernel up to
     8 tokens, split-K cluster kernel up to 64, band kernel from 33 to 1023, 512-row pair tiles from 1024."""
