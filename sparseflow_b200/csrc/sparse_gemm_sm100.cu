@@ -440,7 +440,7 @@ double tile64_cost(int m_tok, int n_out, int K, int num_sms) {
 //   to 32: the 32-token tile, or split K on few row tiles;
 //   33-64: the 64-token tile, four K slices where there are at most a quarter as many row tiles as SMs, the band kernel
 //     (sparse_gemm_sm100_band.cu) where two slices would fit (38-74 row tiles): 8192 x 8192 at 64 tokens 20.8 us split in two,
-//     17.8 us;
+//     17.8 us; two slices where a pair form would have to leave K whole and K is long;
 //   65-128: 64-token tiles or band kernel by estimated time (6000 x 3072 at 72 tokens 8.7 against 10.1 us, 22016 x 4096 29.2
 //     against 26.2);
 //   129-1023: band kernel or fixed tiles by estimated time (bursts: 4096 x 11008 at 150 / 300 tokens 34.6 / 34.4 -> 17.0 / 21.6 us,
@@ -463,6 +463,13 @@ int plan_sparse_gemm(int m_tok, int n_out, int K, int epi, int num_sms) {
   if (m_tok <= 64 && split != 2) return split == 4 ? by_split : 64;
   double band_us = 0.0, fixed_us = 0.0;
   const int band = pick_band_variant(m_tok, n_out, K, num_sms, &band_us);
+  if (m_tok <= 64 && band < 7000) {
+    // Too many row tiles for two pairs each: a split-1 form would stream the weight through half of the pairs, and measured slower than
+    // both alternatives on every shape (8800 x 15552 at 56 tokens: 38.5 us, 64-token tiles 35.3, K split in two 32.9; 8736 x
+    // 6080 at 53 tokens: 19.1, 16.3, 17.5).  Their estimates, fitted to 60 shapes (largest error 0.4 and 0.7 us):
+    const double steps = (K + 127) / 128, hbm = n_out * (K * 1.125) / 6.6e6;
+    return 3.9 + 0.16 * steps + 0.52 * hbm <= 4.5 + 0.081 * steps + 0.625 * hbm + 0.066 * m_tok ? 64 : by_split;
+  }
   if (m_tok <= 128) return tile64_cost(m_tok, n_out, K, num_sms) < band_us ? 64 : band;
   const int fixed = pick_mid_variant(n_out, m_tok, K, num_sms, swiglu, &fixed_us);
   // Those estimates carry 8.5 us outside the K loop, to compare with each other.  Measured as dependent launches it is 3.7 us for the

@@ -307,6 +307,16 @@ def test_small_shapes_keep_the_fixed_tiles():
     assert plan(160, 320, 704, 1) == 6064 and plan(832, 5152, 2944) == 6208 and plan(158, 15232, 4992, 1) == 6160
 
 
+def test_33_to_64_tokens_leave_no_pairs_idle():
+    """Weights with too many row tiles for two pairs each: 64-token tiles, or K split in two where K is long, not pair tiles on half of
+    the pairs (8800 x 15552 at 56 tokens 32.9 against 38.5 us, 8736 x 6080 at 53 tokens 16.3 against 19.1 us)."""
+    from sparseflow_b200 import _lib
+    plan = lambda M, N, K: _lib.lib().sfb200_debug_plan_gemm(M, N, K, 0, 148)
+    assert plan(56, 8800, 15552) == 3064 and plan(59, 9152, 12736) == 3064
+    assert plan(53, 8736, 6080) == 64 and plan(64, 9472, 1024) == 64
+    assert plan(64, 8448, 8192) == 7064 and plan(33, 5184, 5760) == 9048
+
+
 def test_kernel_plan_is_always_a_known_variant():
     """Every shape gets a variant the dispatcher knows, and the families keep to their token ranges: decode kernel up to
     8 tokens, split-K cluster kernel up to 64, band kernel from 33 to 1023, 512-row pair tiles from 1024."""
