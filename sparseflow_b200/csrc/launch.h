@@ -21,9 +21,9 @@
 
 namespace sfb200 {
 
-// cluster = 0: as compiled (none, or __cluster_dims__).
+// cluster = 0: as compiled (none, or __cluster_dims__).  dependent = false: the kernel starts when the one before it has completed.
 template <class... P, class... A>
-int launch_dependent(void (*kernel)(P...), dim3 grid, int block, size_t smem, int cluster, cudaStream_t stream, A&&... args) {
+int launch_kernel(bool dependent, void (*kernel)(P...), dim3 grid, int block, size_t smem, int cluster, cudaStream_t stream, A&&... args) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = grid;
   cfg.blockDim = dim3(static_cast<unsigned>(block), 1, 1);
@@ -32,13 +32,13 @@ int launch_dependent(void (*kernel)(P...), dim3 grid, int block, size_t smem, in
   cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = dependent ? 1 : 0;
   if (cluster > 0) {
-    attr[1].id = cudaLaunchAttributeClusterDimension;
-    attr[1].val.clusterDim.x = static_cast<unsigned>(cluster);
-    attr[1].val.clusterDim.y = 1;
-    attr[1].val.clusterDim.z = 1;
-    cfg.numAttrs = 2;
+    cudaLaunchAttribute& c = attr[cfg.numAttrs++];
+    c.id = cudaLaunchAttributeClusterDimension;
+    c.val.clusterDim.x = static_cast<unsigned>(cluster);
+    c.val.clusterDim.y = 1;
+    c.val.clusterDim.z = 1;
   }
   cfg.attrs = attr;
   if (cudaLaunchKernelEx(&cfg, kernel, std::forward<A>(args)...) != cudaSuccess) {
@@ -46,6 +46,11 @@ int launch_dependent(void (*kernel)(P...), dim3 grid, int block, size_t smem, in
     return kErrCuda;
   }
   return kOk;
+}
+
+template <class... P, class... A>
+int launch_dependent(void (*kernel)(P...), dim3 grid, int block, size_t smem, int cluster, cudaStream_t stream, A&&... args) {
+  return launch_kernel(true, kernel, grid, block, smem, cluster, stream, std::forward<A>(args)...);
 }
 
 }  // namespace sfb200

@@ -370,7 +370,13 @@ int launch_cfg(const SparseGemmArgs& a, cudaStream_t stream) {
   const int tiles = p.num_m_blks * p.num_n_blks;
   int grid = a.num_sms < tiles ? a.num_sms : tiles;
   if (grid < 1) grid = 1;
-  return launch_dependent(sparse_gemm_kernel<C>, grid, 192, C::SMEM_BYTES, 0, stream, tmA, tmB, tmD, p);
+  // A single pass that leaves a quarter of the SMs idle gains little from an early start (its blocks take the idle SMs and wait), and
+  // with few tokens and long K it loses: all blocks then begin to stream at the same moment.  As a dependent launch against a
+  // plain one: 10720 x 5888 at 6 / 11 / 16 tokens 18.8 / 17.7 / 15.3 against 16.8 / 15.8 / 15.7 us, 12448 x 4096 at 6 tokens 14.5 against
+  // 13.8 us; 56 shapes of 75-112 row tiles, 5-14 tokens, K 4096 and 5888: 0.96 on average; with more tiles, more tokens or
+  // K of 1024 and 2048 the dependent launch is the faster one (130 row tiles, 5-14 tokens 0.92).
+  const bool dependent = !(a.m_tok < 16 && 4 * grid <= 3 * a.num_sms && a.K > 3072);
+  return launch_kernel(dependent, sparse_gemm_kernel<C>, grid, 192, C::SMEM_BYTES, 0, stream, tmA, tmB, tmD, p);
 }
 
 // The cheapest, by estimated time, of the single-CTA tiles and the CTA-pair tiles, from 129 to 4095 tokens.  Up to about
