@@ -139,8 +139,7 @@ bool band_has_slices(int m_tok, int n_out, int num_sms, int variant);
 // ---- small-M (decode) sparse GEMM ----------------------------------------------------------
 // Supports M <= 32 tokens; plan_sparse_gemm chooses it for up to 8 (force_bn == 8 forces it).
 int launch_sparse_gemm_small_m(const SparseGemmArgs& a, cudaStream_t stream);
-// Where the split-K cluster kernel applies too (few row tiles): whether this one is the faster, i.e. it has no second, partly
-// filled round of 16-row slabs -- at most one slab per SM, or two blocks per SM with the X cache in shared memory.
+// Where the split-K cluster kernel applies too (few row tiles): whether this one is the faster.
 bool small_m_beats_splitk(int m_tok, int n_out, int K, int num_sms);
 // From 5 tokens the tcgen05 kernel with a 32-token tile is faster (measured); on few row tiles small_m_beats_splitk decides.
 constexpr int kSmallMMaxTokens = 4;

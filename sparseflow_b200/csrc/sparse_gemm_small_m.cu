@@ -369,6 +369,21 @@ int dispatch_nt(const SmallParams& p, int nt, bool bf, int num_sms, cudaStream_t
 
 }  // namespace
 
+// Slabs instead of split K, up to 8 tokens: with the X cache in shared memory, and either one slab per SM or a cache small enough that
+// two blocks would fit an SM and up to four slabs per SM, whether the launch then takes two blocks per SM or one in up to three
+// rounds (297-444 slabs).  Measured, slabs / split K, us (split K as of then, with an early weight prefetch):
+//   rows x K        1 token       2             3             5             8
+//   2048 x  2048     2.8 / 4.5     3.0 / 4.5                                 4.0 / 4.5
+//   4096 x  4096     5.3 / 6.8     6.0 / 6.8     6.6 / 7.1 *   7.0 / 7.2 *   8.4 / 7.2 *
+//   4752 x  1024     3.8 / 5.2     3.7 / 5.1     4.0 / 5.2     4.3 / 5.4     4.0 / 5.2
+//   4752 x  4096     7.5 / 8.8     7.5 / 10.5    8.0 / 10.4 *
+//   5504 x  2048     5.7 / 6.8     5.9 / 6.8     6.3 / 6.8     6.3 / 7.1     6.5 / 6.9 *
+//   7040 x  2048     5.7 / 7.1     6.0 / 7.1     6.4 / 7.1     6.4 / 7.4     6.6 / 7.2 *
+//   7040 x  8192    13.2 / 15.2   13.8 / 14.8 *
+//   8192 x  8192    15.3 / 15.8   17.0 / 17.9 *                             21.8 / 15.8 *
+//   4096 x 11008    11.0 / 11.8   13.6 / 11.8 *                             20.1 / 11.8 *
+//   4096 x 14336    15.3 / 13.9 * 16.6 / 13.9 *                             24.9 / 13.9 *
+// (* = split K by this rule: it keeps a margin where the two are close.)
 bool small_m_beats_splitk(int m_tok, int n_out, int K, int num_sms) {
   if (m_tok > 8 || m_tok * ((K + 127) / 128) > 192) return false;   // (1536 x 4096 at 8 tokens: 6.3 against 5.7 us)
   const int units = (n_out + 15) / 16;
