@@ -42,10 +42,22 @@ WORKLOADS = {
     "llama70b_ffn": (8192, 28672, 8192),
 }
 
-# dram__bytes_read.sum + dram__bytes_write.sum per launch of the gate|up kernel from a profiler capture of the
-# workload itself (`--only gate_up --tokens 4096`, 350 MB on the device): 135.8 MB read + 76.5 MB written, against
-# 225.4 MB algorithmic (part of the output is still in L2 when the kernel ends).
-NCU_TRAFFIC_BYTES = {"llama7b_ffn": 212.4e6}
+# dram__bytes_read.sum + dram__bytes_write.sum per launch of the gate|up kernel from profiler captures of the workload itself
+# (`--only gate_up --tokens 4096`, 350 MB on the device), by workload, tokens and the variant that was captured: 5240 read 146.5 MB and
+# wrote 75.0 MB, 1240 135.8 and 76.5 MB, against 225.4 MB algorithmic (part of the output is still in L2 when the kernel ends).
+NCU_TRAFFIC_BYTES = {("llama7b_ffn", 4096, 5240): 221.5e6, ("llama7b_ffn", 4096, 1240): 212.4e6}
+
+
+def kernel_name(variant):
+    """The kernel a variant number of sfb200_debug_plan_gemm belongs to."""
+    if variant == 8:
+        return "sparse_gemm_small_m_kernel"
+    if variant < 1000:
+        return "sparse_gemm_kernel"
+    if variant >= 6000:
+        return "sparse_gemm_band_kernel"
+    return "sparse_gemm_splitk_kernel" if 3000 <= variant < 5000 else "sparse_gemm_pair_kernel"
+
 
 PARITY_TOL = 1e-2      # FFN output: |d| <= tol * max(|ref|, rms(ref)) and max|d| <= tol * max|ref|
 
@@ -685,10 +697,11 @@ def main():
         peak = 2.0 * burst          # 2:4-sparse rate = 2 x the measured dense bf16 burst figure
         nsm = torch.cuda.get_device_properties(dev).multi_processor_count
         plan = _lib.lib().sfb200_debug_plan_gemm
+        gu_variant = args.tile or plan(M, 2 * I, H, 1, nsm)
         dn_achieved = 2.0 * M * H * I / (dn_ms * 1e-3) / 1e12
         roof = {"bound": "tensor", "achieved": achieved, "peak": peak, "unit": "TFLOP/s",
-                "frac": achieved / peak, "traffic": NCU_TRAFFIC_BYTES.get(args.workload),
-                "kernel": f"sparse_gemm_pair_kernel, SiLU.mul epilogue (gate|up), variant {args.tile or plan(M, 2 * I, H, 1, nsm)}",
+                "frac": achieved / peak, "traffic": NCU_TRAFFIC_BYTES.get((args.workload, M, gu_variant)),
+                "kernel": f"{kernel_name(gu_variant)}, SiLU.mul epilogue (gate|up), variant {gu_variant}",
                 "peak_source": f"2 x bf16_tflops ({src}); of {'measured' if src == 'measured' else 'fallback'}",
                 "frac_of_sustained": achieved / (2.0 * sustained_peak),
                 "ms_per_launch": gu_ms,
@@ -702,8 +715,9 @@ def main():
         gu_ms = tp_phase_ms[0]
         achieved = 2.0 * M * (2 * ffn.Ip) * H / (gu_ms * 1e-3) / 1e12
         peak = 2.0 * burst
+        gu_variant = args.tile or _lib.lib().sfb200_debug_plan_gemm(M, 2 * ffn.Ip, H, 1, torch.cuda.get_device_properties(dev).multi_processor_count)
         roof = {"bound": "tensor", "achieved": achieved, "peak": peak, "unit": "TFLOP/s", "frac": achieved / peak,
-                "traffic": None, "kernel": f"sparse_gemm_pair_kernel, SiLU.mul epilogue (gate|up rows of one rank: {2 * ffn.Ip} x {H})",
+                "traffic": None, "kernel": f"{kernel_name(gu_variant)}, SiLU.mul epilogue (gate|up rows of one rank: {2 * ffn.Ip} x {H}), variant {gu_variant}",
                 "peak_source": f"2 x bf16_tflops ({src}); of {'measured' if src == 'measured' else 'fallback'}; per GPU",
                 "ms_per_launch": gu_ms, "per": "rank, max over ranks, from ten extra steps with events between the phases",
                 "phases_ms": dict(zip(["gate_up_gemm", "down_gemm_and_scatter", "exchange"], tp_phase_ms)),

@@ -39,3 +39,15 @@ def test_repo_arm_fails_loudly_without_a_gpu():
     r = _run("--steps", "1", "--warmup", "1", "--no-cpu-baseline", "--no-parity", "--no-sustained", timeout=300)
     assert r.returncode != 0
     assert not [ln for ln in r.stdout.splitlines() if ln.startswith("{")]      # no benchmark line from a fallback
+
+
+def test_roofline_names_the_kernel_that_runs():
+    """Kernel names by variant number, and the traffic of the default workload is that of the variant a call runs."""
+    sys.path.insert(0, ROOT)
+    import bench
+    from sparseflow_b200 import _lib
+    for variant, name in ((8, "small_m"), (32, "gemm"), (256, "gemm"), (1240, "pair"), (2208, "pair"), (5240, "pair"), (3032, "splitk"),
+                          (4064, "splitk"), (6304, "band"), (9160, "band")):
+        assert bench.kernel_name(variant) == {"gemm": "sparse_gemm_kernel"}.get(name, f"sparse_gemm_{name}_kernel")
+    H, I, M = bench.WORKLOADS["llama7b_ffn"]
+    assert ("llama7b_ffn", M, _lib.lib().sfb200_debug_plan_gemm(M, 2 * I, H, 1, 148)) in bench.NCU_TRAFFIC_BYTES
