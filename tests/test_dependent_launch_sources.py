@@ -18,7 +18,7 @@ DEPENDENT = [f for f in SOURCES if "dependency_wait()" in _code(f)]
 
 
 def test_every_dependent_launch_waits():
-    launching = [f for f in SOURCES if "launch_dependent(" in _code(f)]
+    launching = [f for f in SOURCES if re.search(r"launch_(dependent|kernel)\(", _code(f))]
     assert launching and set(launching) <= set(DEPENDENT)
 
 

@@ -2,7 +2,7 @@
 import pytest
 import torch
 
-from sparseflow_b200 import core, ops, serialize
+from sparseflow_b200 import _lib, core, ops, serialize
 
 pytestmark = pytest.mark.gpu
 
@@ -43,12 +43,20 @@ def test_one_bad_group_is_found(where):
 
 
 def test_forms_outside_the_one_pass_kernel_answer_as_before():
+    """The same error as the separate check and compression, or the verdict of the check."""
     w = torch.zeros(32, 20, device="cuda", dtype=torch.float16)      # K % 16 != 0: no packed form
-    with pytest.raises(Exception):
-        core.compress_2_4(w)
     odd = torch.zeros(33 * 64 + 1, device="cuda", dtype=torch.float16)[1:].view(33, 64)   # unaligned
-    with pytest.raises(Exception):
-        core.compress_2_4(odd)
+    for t, step in ((w, ops.compress_weight), (odd, ops.validate_24)):
+        with pytest.raises(_lib.SfbError) as alone:
+            step(t)
+        with pytest.raises(_lib.SfbError) as checked:
+            core.compress_2_4(t)
+        assert str(checked.value) == str(alone.value)
+    dense = torch.ones(32, 20, device="cuda", dtype=torch.float16)   # not 2:4: found before the width is
+    with pytest.raises(ValueError, match="2:4"):
+        core.compress_2_4(dense)
+    with pytest.raises(ValueError):
+        core.compress_2_4(torch.zeros(32, 64, dtype=torch.float16))  # not on the GPU
 
 
 @pytest.mark.parametrize("rows,K", [(1, 4), (3, 20), (37, 100), (64, 16), (129, 1012), (513, 4092)])

@@ -187,7 +187,7 @@ def test_sparseflow_mlp_module():
     mlp_s = SparseFlowMLP(H, I, to_dev(wg, dt), to_dev(wu, dt), to_dev(wd, dt), down_mode="sparse")
     ref_s = o.ffn_ref(x, pg, pu, pd, dt, round_gate_up=False)["out_f32"]
     assert o.rel_err_metrics(o.to_f32(bits_of(mlp_s(xs)), dt).reshape(96, H), ref_s)["chain"] <= REL_TOL
-    # biases on gate/up take the unfused path
+    # biases on gate/up are added in the epilogue; the reference rounds gate and up to 16 bits before SiLU.mul
     bg, bu = seeded_act(1, I, dt, 11)[0], seeded_act(1, I, dt, 12)[0]
     mlp_b = SparseFlowMLP(H, I, to_dev(wg, dt), to_dev(wu, dt), to_dev(wd, dt), to_dev(bg, dt), to_dev(bu, dt),
                           down_mode="sparse")
