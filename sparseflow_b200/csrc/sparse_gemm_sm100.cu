@@ -445,13 +445,13 @@ double tile64_cost(int m_tok, int n_out, int K, int num_sms) {
 //   1-4 otherwise: the slab kernel;
 //   to 32: the 32-token tile, or split K on few row tiles;
 //   33-64: the 64-token tile, four K slices where there are at most a quarter as many row tiles as SMs, the band kernel
-//     (sparse_gemm_sm100_band.cu) where two slices would fit (38-74 row tiles): 8192 x 8192 at 64 tokens 20.8 us split in two,
-//     17.8 us; two slices where a pair form would have to leave K whole and K is long;
+//     (sparse_gemm_sm100_band.cu) where two slices would fit (38-74 row tiles): 8192 x 8192 at 64 tokens 21.8 us split in two,
+//     18.3 us; two slices where a pair form would have to leave K whole and K is long;
 //   65-128: 64-token tiles or band kernel by estimated time (6000 x 3072 at 72 tokens 8.7 against 10.1 us, 22016 x 4096 29.2
 //     against 26.2);
-//   129-1023: band kernel or fixed tiles by estimated time (bursts: 4096 x 11008 at 150 / 300 tokens 34.6 / 34.4 -> 17.0 / 21.6 us,
-//     22016 x 4096 32.8 / 42.1 -> 25.2 / 32.6 us; steady: 8192 x 8192 at 520 tokens 55.5 -> 42.0 us; at 700-1000 tokens and on small
-//     shapes the two meet).  On 400 random shapes (256-24000 rows, K 512-12288) the choice averages 1.01 of the faster of the two;
+//   129-1023: band kernel or fixed tiles by estimated time (steady load: 4096 x 11008 at 150 / 300 tokens 33.6 / 34.0 -> 17.8 /
+//     23.6 us, 22016 x 4096 33.0 / 47.3 -> 28.8 / 38.4 us, 8192 x 8192 at 520 tokens 56.2 -> 42.5 us; at 700-1000 tokens and on
+//     small shapes the two meet).  On 400 random shapes (256-24000 rows, K 512-12288) the choice averages 1.01 of the faster of the two;
 //   from 1024: pair or single-CTA tiles, to 4095 by estimated time, above that pair tiles; a 512-row tile in place of a
 //     256-row one with two accumulator sets where pick_pair_variant_sustained prefers it.
 int plan_sparse_gemm(int m_tok, int n_out, int K, int epi, int num_sms) {

@@ -20,9 +20,9 @@
 //     bytes per store instruction, and the owner adds them in pair order.  No scratch in global memory, no
 //     atomics, the same bits on every run.
 //
-// Measured (B200, steady load at the power limit, fixed tiles before -> now): 4096 x 11008 at 150 / 300 / 400 tokens 34.2 / 34.2 /
-// 36.2 -> 18.5 / 24.3 / 28.0 us; 22016 x 4096 (SiLU.mul) at 72 / 150 / 300 / 400 tokens 27.9 / 33.1 / 47.8 / 49.1 -> 25.5 / 28.3 /
-// 36.9 / 44.5 us; 8192 x 8192 at 520 tokens 55.5 -> 42.0 us; 57344 x 8192 at 300 tokens 219.7 -> 176.8 us.  Evict-last token loads and
+// Measured (B200, steady load at the power limit, fixed tiles before -> now): 4096 x 11008 at 150 / 300 / 400 tokens 33.6 / 34.0 /
+// 35.9 -> 17.8 / 23.6 / 28.2 us; 22016 x 4096 (SiLU.mul) at 72 / 150 / 300 / 400 tokens 28.3 / 33.0 / 47.3 / 50.1 -> 24.8 / 28.8 /
+// 38.4 / 43.3 us; 8192 x 8192 at 520 tokens 56.2 -> 42.5 us; 57344 x 8192 at 300 tokens 211 -> 171 us.  90 registers, no spills.  Evict-last token loads and
 // evict-first stores are 3-10 % of that.  Split 3 against split 2: 4096 x 11008 at 96 / 150 tokens 18.3 / 19.2 -> 16.0 / 17.6 us.
 //
 // Warps: warp 0 = TMA producer, warp 1 = MMA issuer / tensor-memory owner, warps 2 ... 17 = epilogue.
