@@ -451,7 +451,7 @@ double tile64_cost(int m_tok, int n_out, int K, int num_sms) {
 //     against 26.2);
 //   129-1023: band kernel or fixed tiles by estimated time (steady load: 4096 x 11008 at 150 / 300 tokens 33.6 / 34.0 -> 17.8 /
 //     23.6 us, 22016 x 4096 33.0 / 47.3 -> 28.8 / 38.4 us, 8192 x 8192 at 520 tokens 56.2 -> 42.5 us; at 700-1000 tokens and on
-//     small shapes the two meet).  On 400 random shapes (256-24000 rows, K 512-12288) the choice averages 1.01 of the faster of the two;
+//     small shapes the two meet).  On 400 random shapes (256-24000 rows, K 512-12288) the choice averages 1.011 of the faster of the two;
 //   from 1024: pair or single-CTA tiles, to 4095 by estimated time, above that pair tiles; a 512-row tile in place of a
 //     256-row one with two accumulator sets where pick_pair_variant_sustained prefers it.
 int plan_sparse_gemm(int m_tok, int n_out, int K, int epi, int num_sms) {
@@ -482,13 +482,13 @@ int plan_sparse_gemm(int m_tok, int n_out, int K, int epi, int num_sms) {
   // single-CTA tiles (median of 204 shapes; 4.2 where they meet the band kernel) and, at short K, 5.6 us for the pair tiles (126 shapes);
   // with 8.5 the band kernel was taken on small shapes where it is the slower one (2240 x 768 at 850 tokens 7.5 against 5.9 us, 8000 x 512 at
   // 239 tokens 6.8 against 5.3, 9536 x 832 with SiLU.mul at 630 tokens 11.9 against 10.8).
-  if (fixed < 256) fixed_us -= 8.5 - 4.2;
-  else if (K <= 1408) fixed_us -= 8.5 - 5.6;
+  const bool lowered = fixed < 256 || K <= 1408;
+  if (lowered) fixed_us -= 8.5 - (fixed < 256 ? 4.2 : 5.6);
   // The same tile as the fixed kernel's, with no left-over tiles to slice, has nothing to gain (2-4 % slower).  Above 800
-  // tokens the estimate is trusted by a wider margin: there the tiles with a single accumulator set fall behind it
-  // (8192 x 28672 at 1000 tokens estimated 0.95, measured 1.17 of the fixed tile).
+  // tokens the estimate is trusted by a margin: there the tiles with a single accumulator set fall behind it (8192 x 28672 at
+  // 1000 tokens estimated 0.95, measured 1.17 of the fixed tile; 7456 x 5312 with SiLU.mul at 1009 tokens 0.89 and 1.05).
   if (band % 1000 == fixed % 1000 && fixed >= 1000 && fixed < 3000 && !band_has_slices(m_tok, n_out, num_sms, band)) return fixed;
-  return band_us < (m_tok > 800 ? 0.9 : 1.0) * fixed_us ? band : fixed;
+  return band_us < (m_tok <= 800 ? 1.0 : lowered ? 0.9 : 0.8) * fixed_us ? band : fixed;
 }
 
 int launch_sparse_gemm(const SparseGemmArgs& a, cudaStream_t stream) {

@@ -304,6 +304,7 @@ def test_small_shapes_keep_the_fixed_tiles():
     plan = lambda M, N, K, sw=0: _lib.lib().sfb200_debug_plan_gemm(M, N, K, sw, 148)
     assert plan(850, 2240, 768) == 128 and plan(461, 4448, 768) == 128 and plan(239, 8000, 512) == 128
     assert plan(623, 2880, 1280) == 128 and plan(133, 7872, 832) == 128 and plan(630, 9536, 832, 1) == 1224
+    assert plan(1009, 7456, 5312, 1) == 1256              # above 800 tokens an estimate of 0.9 of the fixed tile is not enough
     assert plan(160, 320, 704, 1) == 6064 and plan(832, 5152, 2944) == 6208 and plan(158, 15232, 4992, 1) == 6160
 
 
